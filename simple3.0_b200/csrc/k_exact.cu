@@ -5,7 +5,8 @@
 // (calc_corr_for_rot, simple_polarft_corrcalc.f90:1190-1216, with ptcl~ the
 // particle extended over the full circle by conjugate symmetry), for every
 // rotation at once, with the reference prepared exactly as gencorrs_cc_1/_2 do
-// (prep_ref4corr :961-985, gen_shmat_8 :1098-1120, :1526-1531).
+// (prep_ref4corr :961-985, gen_shmat_8 :1098-1120, :1526-1531).  They serve the numbers of
+// rotations that k_exact_fft.cu has no transform for.
 #include "pftcc_internal.cuh"
 
 #include <cstddef>
@@ -436,9 +437,15 @@ static cudaError_t launch_exact_t(pftcc_handle *h, int kc, size_t smem, const Gr
 }
 
 cudaError_t launch_exact(pftcc_handle *h, const Group *groups, int ngroups, const Work *work, const float *shifts,
-                         int mode, int frame, int cc1_kstop, float *out, pftcc_best *best, const uint8_t *rotmask)
+                         int mode, int frame, int cc1_kstop, int max_items, float *out, pftcc_best *best,
+                         const uint8_t *rotmask)
 {
     if (frame == FRAME_EUCLID && (!h->d_sig2 || !h->d_pxls)) return cudaErrorInvalidValue;
+    // the transforms wherever their lengths allow (tens of times fewer operations, no size at which the
+    // direct sums were faster); the direct sums serve the other numbers of rotations
+    if (exact_fft_supported(h->g.P))
+        return launch_exact_fft(h, groups, ngroups, work, shifts, mode, frame, cc1_kstop, max_items, out, best, rotmask,
+                                nullptr);
     size_t smem;
     const int kc = exact_kc(h->g, frame, &smem);
     if (frame == PFTCC_FRAME_PTCL)

@@ -1471,7 +1471,7 @@ int search_mdomain(pftcc_handle *h, int nshifts_in, const float *shifts_host, in
     k_finish<<<(np + 127) / 128, 128, 0, h->stream>>>(ws.cand, d_perm, np, N, ns, nshifts_in > 0, ntop, out_dev,
                                                       h->d_work, h->d_groups);
     CKE(cudaGetLastError(), "finish");
-    CKE(launch_exact(h, h->d_groups, np, h->d_work, ws.shifts, MODE_BEST, exact_frame(h), 1, nullptr, out_dev),
+    CKE(launch_exact(h, h->d_groups, np, h->d_work, ws.shifts, MODE_BEST, exact_frame(h), 1, ntop, nullptr, out_dev),
         "rescore");
 #undef CKE
     return PFTCC_OK;
@@ -1760,7 +1760,7 @@ int search_mdomain_groups(pftcc_handle *h, int ngroups, const int *ref0, const i
             k_finish<<<(bt.n + 127) / 128, 128, 0, h->stream>>>(ws.cand, bperm, bt.n, N, ns, nshifts_in > 0, ntop,
                                                                 out_dev, h->d_work, h->d_groups);
             CKG(cudaGetLastError(), "finish");
-            CKG(launch_exact(h, h->d_groups, bt.n, h->d_work, ws.shifts, MODE_BEST, exact_frame(h), 1, nullptr,
+            CKG(launch_exact(h, h->d_groups, bt.n, h->d_work, ws.shifts, MODE_BEST, exact_frame(h), 1, ntop, nullptr,
                              out_dev),
                 "rescore");
         }

@@ -131,7 +131,7 @@ static int corr_all_device(pftcc_handle *h, int precision, float *dst)
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(h->d_groups, groups.data(), m * sizeof(Group), cudaMemcpyHostToDevice, h->stream);
         if (e == cudaSuccess)
-            e = launch_exact(h, h->d_groups, m, h->d_work, nullptr, MODE_FULL, exact_frame(h), 1,
+            e = launch_exact(h, h->d_groups, m, h->d_work, nullptr, MODE_FULL, exact_frame(h), 1, h->nrefs,
                              dst + (size_t)c0 * per_ptcl * h->g.N, nullptr);
         if (e != cudaSuccess) return cuda_err(h, e, "snhc correlations");
     }

@@ -96,7 +96,7 @@ extern "C" int pftcc_gencorrs_noalloc(pftcc_handle *h, int npairs, const int *ir
     const Work *dw = reinterpret_cast<const Work *>(b);
     const Group *dg = reinterpret_cast<const Group *>(b + (size_t)npairs * sizeof(Work));
     const float *ds = reinterpret_cast<const float *>(b + (size_t)npairs * (sizeof(Work) + sizeof(Group)));
-    e = launch_exact(h, dg, npairs, dw, ds, MODE_FULL, exact_frame(h), 1, cc_dev, nullptr);
+    e = launch_exact(h, dg, npairs, dw, ds, MODE_FULL, exact_frame(h), 1, 1, cc_dev, nullptr);
     if (e != cudaSuccess) return cuda_err(h, e, "gencorrs_noalloc kernel");
     // the host descriptors must outlive the copy
     e = cudaStreamSynchronize(h->stream);

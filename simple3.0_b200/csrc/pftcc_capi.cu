@@ -306,7 +306,7 @@ static int build_polarizer(pftcc_handle *h, int griddev)
 static void free_all(pftcc_handle *h)
 {
     void *ptrs[] = {h->refs_even, h->refs_odd, h->ptcls, h->sqsums, h->ctfmats, h->d_iseven, h->d_ctfp, h->polar,
-                    h->argtransf, h->argtransf1, h->pol_off, h->pol_w, h->pol_stage, h->d_work, h->d_groups,
+                    h->argtransf, h->argtransf1, h->d_wn, h->d_expart, h->pol_off, h->pol_w, h->pol_stage, h->d_work, h->d_groups,
                     h->d_out, h->d_shifts, h->d_dout, h->d_best, h->ws.UA, h->ws.UB, h->ws.RU, h->ws.CV,
                     h->ws.RUf, h->ws.CVf, h->ws.D, h->ws.Yn, h->ws.X, h->ws.cand, h->ws.sqp, h->ws.A16, h->ws.B16, h->ws.shifts, h->ws.best,
                     h->ws.cand_ref, h->vol_cube, h->d_sig2, h->d_pxls, h->drefs_even, h->drefs_odd, h->d_optlp,
@@ -319,6 +319,7 @@ static void free_all(pftcc_handle *h)
     cudaStream_t own = h->own_stream ? h->own_stream : h->stream;
     if (own) cudaStreamDestroy(own);
     for (void *&p : h->pin) { if (p) cudaFreeHost(p); p = nullptr; }
+    if (h->pin_cc) cudaFreeHost(h->pin_cc);
 }
 
 static int alloc_ptcl_arrays(pftcc_handle *h)
@@ -429,9 +430,16 @@ int pftcc_new(const pftcc_config *cfg, const int *ptcl_mask, const int *eoarr, p
         (st = dev_alloc(h, (void **)&h->polar, h->h_polar.size() * sizeof(float), "polar")) ||
         (st = dev_alloc(h, (void **)&h->argtransf, h->h_argtransf.size() * sizeof(double), "argtransf")) ||
         (st = dev_alloc(h, (void **)&h->argtransf1, h->h_argtransf1.size() * sizeof(double), "argtransf1")) ||
+        (st = dev_alloc(h, (void **)&h->d_wn, (size_t)h->g.N * sizeof(double2), "twiddles")) ||
         (st = alloc_ptcl_arrays(h)))
         return fail(st, h->last_err);
-    if (cudaMemsetAsync(h->refs_even, 0, (size_t)h->nrefs * KP * sizeof(float2), h->stream) ||
+    std::vector<double2> wn(h->g.N);
+    for (int e = 0; e < h->g.N; ++e) {
+        const double a = -2.0 * M_PI * e / h->g.N;
+        wn[e] = make_double2(cos(a), sin(a));
+    }
+    if (cudaMemcpyAsync(h->d_wn, wn.data(), wn.size() * sizeof(double2), cudaMemcpyHostToDevice, h->stream) ||
+        cudaMemsetAsync(h->refs_even, 0, (size_t)h->nrefs * KP * sizeof(float2), h->stream) ||
         cudaMemsetAsync(h->refs_odd, 0, (size_t)h->nrefs * KP * sizeof(float2), h->stream) ||
         cudaMemcpyAsync(h->polar, h->h_polar.data(), h->h_polar.size() * sizeof(float), cudaMemcpyHostToDevice,
                         h->stream) ||
@@ -1245,13 +1253,25 @@ static int gencorrs_frame(pftcc_handle *h, int iref, int iptcl, const float *shv
 {
     REF_OR_FAIL(iref);
     SLOT_OR_FAIL(slot, iptcl);
+    if (exact_fft_supported(h->g.P)) {
+        // one launch and one wait: the request goes as the kernel's argument and the kernel writes its N
+        // values to pinned memory (three uploads and a download were half of such a call)
+        if (frame == FRAME_EUCLID && (!h->d_sig2 || !h->d_pxls)) return set_err(h, PFTCC_ERR_STATE, "gencorrs: no sigma2");
+        if (!h->pin_cc) CK(cudaMallocHost((void **)&h->pin_cc, h->g.N * sizeof(float)), "gencorrs");
+        const ExactOne one{iref - 1, slot, shvec ? 1 : 0, shvec ? shvec[0] : 0.f, shvec ? shvec[1] : 0.f};
+        CK(launch_exact_fft(h, nullptr, 1, nullptr, nullptr, MODE_FULL, frame, 1, 1, h->pin_cc, nullptr, nullptr, &one),
+           "gencorrs kernel");
+        CK(cudaStreamSynchronize(h->stream), "gencorrs");
+        std::memcpy(cc, h->pin_cc, h->g.N * sizeof(float));
+        return PFTCC_OK;
+    }
     ST(ensure_small(h, 1, 1, h->g.N, 1));
     Work w{iref - 1, shvec ? 0 : -1, 0};
     Group gr{slot, 0, 1, 0};
     CK(cudaMemcpyAsync(h->d_work, &w, sizeof(w), cudaMemcpyHostToDevice, h->stream), "gencorrs");
     CK(cudaMemcpyAsync(h->d_groups, &gr, sizeof(gr), cudaMemcpyHostToDevice, h->stream), "gencorrs");
     if (shvec) CK(cudaMemcpyAsync(h->d_shifts, shvec, 2 * sizeof(float), cudaMemcpyHostToDevice, h->stream), "gencorrs");
-    CK(launch_exact(h, h->d_groups, 1, h->d_work, h->d_shifts, MODE_FULL, frame, 1, h->d_out, nullptr),
+    CK(launch_exact(h, h->d_groups, 1, h->d_work, h->d_shifts, MODE_FULL, frame, 1, 1, h->d_out, nullptr),
        "gencorrs kernel");
     CK(cudaMemcpyAsync(cc, h->d_out, h->g.N * sizeof(float), cudaMemcpyDeviceToHost, h->stream), "gencorrs");
     CK(cudaStreamSynchronize(h->stream), "gencorrs");
@@ -1606,7 +1626,7 @@ int pftcc_calc_roinv_corrmat(pftcc_handle *h, float *corrmat)
         CK(cudaMemcpyAsync(h->d_work, work.data(), wi * sizeof(Work), cudaMemcpyHostToDevice, h->stream), "corrmat");
         CK(cudaMemcpyAsync(h->d_groups, groups.data(), groups.size() * sizeof(Group), cudaMemcpyHostToDevice, h->stream),
            "corrmat");
-        CK(launch_exact(h, h->d_groups, (int)groups.size(), h->d_work, nullptr, MODE_ITEMMAX, exact_frame(h), 1,
+        CK(launch_exact(h, h->d_groups, (int)groups.size(), h->d_work, nullptr, MODE_ITEMMAX, exact_frame(h), 1, n - 1,
                         h->d_out, nullptr), "corrmat kernel");
         std::vector<float> mx(npairs);
         CK(cudaMemcpyAsync(mx.data(), h->d_out, npairs * sizeof(float), cudaMemcpyDeviceToHost, h->stream), "corrmat");
@@ -1652,7 +1672,7 @@ int pftcc_corr_all(pftcc_handle *h, int nshifts, const float *shifts, float *cc)
         }
         CK(cudaMemcpyAsync(h->d_work, work.data(), wi * sizeof(Work), cudaMemcpyHostToDevice, h->stream), "work");
         CK(cudaMemcpyAsync(h->d_groups, groups.data(), m * sizeof(Group), cudaMemcpyHostToDevice, h->stream), "groups");
-        CK(launch_exact(h, h->d_groups, m, h->d_work, h->d_shifts, MODE_FULL, exact_frame(h), 1, h->d_out, nullptr),
+        CK(launch_exact(h, h->d_groups, m, h->d_work, h->d_shifts, MODE_FULL, exact_frame(h), 1, (int)per_ptcl, h->d_out, nullptr),
            "corr_all kernel");
         CK(cudaMemcpyAsync(cc + (size_t)c0 * out_per_ptcl, h->d_out, (size_t)m * out_per_ptcl * sizeof(float),
                            cudaMemcpyDeviceToHost, h->stream), "corr_all download");
@@ -1697,7 +1717,7 @@ static int search_exact(pftcc_handle *h, int nshifts, const float *shifts, pftcc
     CK(cudaMemcpyAsync(h->d_work, work.data(), wi * sizeof(Work), cudaMemcpyHostToDevice, h->stream), "work");
     CK(cudaMemcpyAsync(h->d_groups, groups.data(), groups.size() * sizeof(Group), cudaMemcpyHostToDevice, h->stream),
        "groups");
-    CK(launch_exact(h, h->d_groups, h->nptcls, h->d_work, h->d_shifts, MODE_BEST, exact_frame(h), 1, nullptr, out_dev),
+    CK(launch_exact(h, h->d_groups, h->nptcls, h->d_work, h->d_shifts, MODE_BEST, exact_frame(h), 1, (int)per_ptcl, nullptr, out_dev),
        "search exact");
     return PFTCC_OK;
 }

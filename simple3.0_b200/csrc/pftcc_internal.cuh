@@ -143,6 +143,7 @@ struct pftcc_handle {
     int ctf_ready = 0;
     float *polar = nullptr;
     double *argtransf = nullptr, *argtransf1 = nullptr;
+    double2 *d_wn = nullptr;             // w_N^{-e} = exp(-2 pi i e / N), e < N
     std::vector<float> h_polar;
     std::vector<double> h_argtransf, h_argtransf1;
     std::vector<float> angtab;           // degrees
@@ -183,6 +184,9 @@ struct pftcc_handle {
     size_t shifts_cap = 0;
     double *d_dout = nullptr;
     size_t dout_cap = 0;
+    void *d_expart = nullptr;            // the exact search's partial results (k_exact_fft.cu)
+    size_t expart_cap = 0;
+    float *pin_cc = nullptr;             // [N] pinned: one gencorrs call's result, written by its kernel
     pftcc_best *d_best = nullptr;
     size_t best_cap = 0;
     pftcc::SearchWS ws;
@@ -251,11 +255,18 @@ cudaError_t launch_fdf_project_polar(pftcc_handle *h, int box, const float2 *cub
 cudaError_t launch_ctfmat(pftcc_handle *h, const pftcc_ctfparams *params, int n, float *out, float ddf,
                           int derivative);
 cudaError_t launch_sqsums(pftcc_handle *h, int first_slot, int n);
-// rotmask (optional) [ngroups][N]: MODE_BEST / MODE_ITEMMAX take their maxima over the
-// rotations whose mask byte is non-zero
+// max_items: the most work items any of the groups has.  rotmask (optional) [ngroups][N]: MODE_BEST /
+// MODE_ITEMMAX take their maxima over the rotations whose mask byte is non-zero
 cudaError_t launch_exact(pftcc_handle *h, const Group *groups, int ngroups, const Work *work,
-                         const float *shifts, int mode, int frame, int cc1_kstop, float *out,
+                         const float *shifts, int mode, int frame, int cc1_kstop, int max_items, float *out,
                          pftcc_best *best, const uint8_t *rotmask = nullptr);
+// the same by FP64 transforms (k_exact_fft.cu) for the lengths exact_fft_supported names; `one` instead
+// of the tables for a single correlation (MODE_FULL, out[0..N-1])
+struct ExactOne { int iref, slot, has_shift; float sx, sy; };   // iref 0-based
+bool exact_fft_supported(int P);
+cudaError_t launch_exact_fft(pftcc_handle *h, const Group *groups, int ngroups, const Work *work, const float *shifts,
+                             int mode, int frame, int cc1_kstop, int max_items, float *out, pftcc_best *best,
+                             const uint8_t *rotmask, const ExactOne *one);
 // single-rotation correlation requests for k_for_rot: iref 0-based, slot, irot 1-based,
 // ctf_mode 0 = the stored |CTF| matrices (the drop-in calls), 1 = |CTF| recomputed at
 // defocus + ddf; out5 [n][5] = f, df/dsx, df/dsy, df/ddf, unused

@@ -305,9 +305,11 @@ int shsrch_batch(pftcc_handle *h, int mode, const pftcc_shsrch_opts &o, int n, c
             groups.clear();
             shifts.clear();
             bool any_mask = false;
+            int most = 1;
             for (int b = 0; b < ng; ++b) {
                 Problem &p = pr[who_scan[b]];
                 const int ns = (int)p.sc.size() / 2;
+                most = std::max(most, ns);
                 p.scan_base = (int)(shifts.size() / 2);
                 groups.push_back(Group{p.slot, (int)work.size(), ns, b});
                 for (int s = 0; s < ns; ++s) work.push_back(Work{p.iref0, (int)(shifts.size() / 2) + s, 0});
@@ -338,7 +340,7 @@ int shsrch_batch(pftcc_handle *h, int mode, const pftcc_shsrch_opts &o, int n, c
                 (any_mask && (e = cudaMemcpyAsync(dmask, gmask.data(), mbytes, cudaMemcpyHostToDevice, h->stream)) !=
                                  cudaSuccess))
                 return cuda_err(h, e, "shsrch upload");
-            if ((e = launch_exact(h, h->d_groups, ng, h->d_work, h->d_shifts, MODE_BEST, exact_frame(h), 1, nullptr,
+            if ((e = launch_exact(h, h->d_groups, ng, h->d_work, h->d_shifts, MODE_BEST, exact_frame(h), 1, most, nullptr,
                                   h->d_best, dmask)) != cudaSuccess)
                 return cuda_err(h, e, "shsrch gencorrs");
             bres.resize(ng);

@@ -22,7 +22,8 @@ __device__ __forceinline__ double2 d_add(double2 a, double2 b) { return make_dou
 __device__ __forceinline__ double2 d_sub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 d_mul(double2 a, double2 b)
 {
-    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+    // rounded products, so that no caller's inlining contracts them differently
+    return make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
 
 // forward radix butterflies (the textbook radix-2/3/4/5 DFT formulas), FP64
@@ -62,8 +63,8 @@ template <> struct DBfly<5> {
         const double2 t3 = d_sub(v[1], v[4]), t4 = d_sub(v[2], v[3]);
         const double2 m1 = make_double2(fma(c2, t2.x, fma(c1, t1.x, a.x)), fma(c2, t2.y, fma(c1, t1.y, a.y)));
         const double2 m2 = make_double2(fma(c1, t2.x, fma(c2, t1.x, a.x)), fma(c1, t2.y, fma(c2, t1.y, a.y)));
-        const double2 n1 = make_double2(fma(s2, t4.x, s1 * t3.x), fma(s2, t4.y, s1 * t3.y));
-        const double2 n2 = make_double2(fma(-s1, t4.x, s2 * t3.x), fma(-s1, t4.y, s2 * t3.y));
+        const double2 n1 = make_double2(fma(s2, t4.x, __dmul_rn(s1, t3.x)), fma(s2, t4.y, __dmul_rn(s1, t3.y)));
+        const double2 n2 = make_double2(fma(-s1, t4.x, __dmul_rn(s2, t3.x)), fma(-s1, t4.y, __dmul_rn(s2, t3.y)));
         v[0] = d_add(d_add(a, t1), t2);
         v[1] = make_double2(m1.x + n1.y, m1.y - n1.x);   // m1 - i n1
         v[4] = make_double2(m1.x - n1.y, m1.y + n1.x);

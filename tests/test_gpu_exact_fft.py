@@ -1,0 +1,81 @@
+"""GPU tests of the exact correlations by transforms (the lengths 64, 180 and 300): every correlation
+against the FP64 oracle at the edges of the kernel's shell pairs, item chunks and modes, and the same
+bits for a request alone, in a batch and in a search.
+
+Tolerance without a CTF: the operands are the reference times the shift phase in FP32 -- the phase's
+rounding and the complex product's, at most 4 half-ulps (2^-24) of each sample's modulus -- so by
+Cauchy-Schwarz a correlation of unit vectors moves by at most 4 * 2^-24 = 2.4e-7; the FP32 square sum
+of the particle (a few 1e-8 relative) and the result's rounding (6e-8) leave 4e-7."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+TOL = 4e-7
+
+
+def build(pkg, name, nrefs, nptcls, frame, kstop=None, ctf=False, kto=None):
+    w = getattr(pkg.synth, name)(nrefs=nrefs, nptcls=nptcls)
+    if kto:
+        w.kto = kto
+    refs, R = pkg.synth.make_refs(w)
+    parts = pkg.synth.make_particles(w, R)
+    pc = pkg.polarft_corrcalc()
+    pc.new(nrefs, (1, nptcls), box=w.box, nrots=w.nrots, kfromto=(w.kfrom, w.kto), kstop=kstop, ctf=ctf, ctf_frame=frame,
+           eoarr=[0] * nptcls)
+    pc.set_refs(1, refs.numpy(), True)
+    pc.polarize_ptcls(0, parts.cmat.numpy())
+    if ctf:
+        pc.create_polar_absctfmats(pkg.ctfparams_array(nptcls, smpd=w.smpd, kv=w.kv, cs=w.cs, fraca=w.fraca,
+                                                       dfx=parts.dfx, dfy=parts.dfy, angast=parts.angast))
+    return w, pc, refs.numpy()
+
+
+@pytest.mark.parametrize("frame", ["ref", "ptcl"])
+@pytest.mark.parametrize("name,kstop", [("config0", 20), ("config0", 2), ("config0", 9), ("config1", 40), ("config1", 37),
+                                        ("geometry_c", 60), ("geometry_c", 55)])
+def test_every_correlation(pkg, O, name, kstop, frame):
+    """odd and even shell counts, one shell, shells beyond kstop; 5 references = a chunk and a remainder"""
+    w, pc, refs = build(pkg, name, 5, 3, frame, kstop=kstop)
+    g = O.geom(w.nrots, w.kfrom, w.kto, w.box, kstop=kstop)
+    ptcls = np.stack([pc.get_ptcl_pft(i + 1) for i in range(3)])
+    for shifts in (None, np.array([[0.0, 0.0], [1.5, -0.75], [-2.0, 2.0]], np.float32)):
+        want = O.allcorrs64(g, O.tables(g), refs, ptcls, None, shifts, frame)
+        assert np.max(np.abs(pc.corr_all(shifts) - want)) < TOL
+    pc.kill()
+
+
+@pytest.mark.parametrize("name", ["config0", "config1", "geometry_c"])
+@pytest.mark.parametrize("frame", ["ref", "ptcl"])
+@pytest.mark.parametrize("nrefs,nptcls,ns", [(1, 3, 0), (2, 3, 1), (3, 2, 1), (4, 2, 2), (9, 2, 1), (21, 1, 2), (7, 40, 1)])
+def test_batch_and_search_equal_single_calls(pkg, name, frame, nrefs, nptcls, ns):
+    """1 to 42 items a particle: a single item, chunks, a particle's items shared between blocks"""
+    if name != "config0" and nptcls > 10:
+        nptcls = 12
+    w, pc, refs = build(pkg, name, nrefs, nptcls, frame, ctf=True, kto=11)
+    shifts = None if ns == 0 else np.array([[0.5, -1.0], [-1.0, 0.25]], np.float32)[:ns]
+    cc = pc.corr_all(shifts)
+    for i in (0, nptcls - 1):
+        for r in (0, nrefs - 1):
+            for s in range(max(1, ns)):
+                assert np.array_equal(cc[i, r, s], pc.gencorrs(r + 1, i + 1, None if ns == 0 else shifts[s]))
+    best = pc.search_best(shifts, "exact")
+    flat = cc.reshape(nptcls, -1).argmax(1)
+    assert np.array_equal(best["corr"], cc.reshape(nptcls, -1).max(1))
+    assert np.array_equal(best["iref"] - 1, flat // (max(1, ns) * w.nrots))
+    assert np.array_equal(best["irot"] - 1, flat % w.nrots)
+    pc.kill()
+
+
+def test_zero_reference_is_never_the_best(pkg):
+    """0 / 0 is not a number and takes no part in a maximum, as with the direct sums"""
+    w, pc, refs = build(pkg, "config0", 3, 2, "ptcl", ctf=True)
+    zero = refs.copy()
+    zero[1] = 0
+    pc.set_refs(1, zero, True)
+    cc = pc.corr_all(None)
+    assert np.all(np.isnan(cc[:, 1])) and np.all(np.isfinite(cc[:, [0, 2]]))
+    assert np.all(pc.search_best(None, "exact")["iref"] != 2)
+    pc.set_refs(1, np.zeros_like(refs), True)
+    best = pc.search_best(None, "exact")
+    assert np.all(best["iref"] == 0) and np.all(best["irot"] == 0) and np.all(np.isneginf(best["corr"]))
+    pc.kill()
