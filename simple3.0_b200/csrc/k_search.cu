@@ -41,11 +41,10 @@ namespace pftcc {
 int umma_stage1(pftcc_handle *h, int M, int Ks, const float2 *UA, int rs0, int nrs_w, int rows_pad,
                 const float2 *UB, int c0, int ncols_w, int cols_pad, float2 *X, int prepare, int parity_group);
 bool stage2_fast_supported(int P);
-int stage2_fast_p2(int P);
 int stage2_fast_dlen(int P);
 cudaError_t launch_stage2_fast(pftcc_handle *h, int P, int rows, int xrows, int xcols, int row0, int nshifts, int r0,
                                int dcols, int col0, int cols, int nrs_total, const float2 *X, const float *Dinv,
-                               float2 *cand, float *ccall, const int *perm, int eu);
+                               float2 *cand, float *ccall, const int *perm, int eu, int rot);
 cudaError_t launch_rescore_md(pftcc_handle *h, int P, int ncols, int ntop, int Ks, int nshifts, int has_shifts,
                               const float2 *UA, int rows_pad, const float2 *UB, int cols_pad, const double2 *RU,
                               const double2 *CV, const float *sqp, const float2 *cand, const int *perm, int c0,
@@ -550,7 +549,7 @@ constexpr int COL_TILE = 128;
 
 __global__ void __launch_bounds__(256) k_stage1_fp32(int Ks, int P, const float2 *__restrict__ UA, int rows_pad,
                                                      int row0, const float2 *__restrict__ UB, int cols_pad, int col0,
-                                                     float2 *__restrict__ Z, int xrows, int xcols)
+                                                     float4 *__restrict__ Z, int xrows, int xcols)
 {
     extern __shared__ float4 smem4[];
     float2 *sa = reinterpret_cast<float2 *>(smem4);   // [2 planes][Ks][64] rows
@@ -599,24 +598,31 @@ __global__ void __launch_bounds__(256) k_stage1_fp32(int Ks, int P, const float2
     }
     const int N = 2 * P;
     const float2 wA = wn_of(mA, N), wB = wn_of(mB, N);
+    const size_t half = (size_t)(xrows >> 1);   // row pairs of a column
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int col = ct + 4 * ty + j;
         if (col >= xcols) continue;
-        float2 *dA = Z + ((size_t)mA * xcols + col) * xrows + rt + 4 * tx;
-        float2 *dB = Z + ((size_t)(mB < P ? mB : 0) * xcols + col) * xrows + rt + 4 * tx;
+        float4 *dA = Z + ((size_t)mA * xcols + col) * half + (rt >> 1) + 2 * tx;
+        float4 *dB = Z + ((size_t)(mB < P ? mB : 0) * xcols + col) * half + (rt >> 1) + 2 * tx;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 4; i += 2) {
             if (rt + 4 * tx + i >= xrows) continue;
-            float2 xa = make_float2(4.f * accr[0][i][j], 4.f * acci[0][i][j]);
-            float2 xb = make_float2(4.f * accr[1][i][j], 4.f * acci[1][i][j]);
-            if (mp == 0) {              // X(0) and X(P) are real
-                xa.y = 0.f;
-                xb.y = 0.f;
-                dA[i] = make_z(xa, xb, wA);
-            } else {
-                dA[i] = make_z(xa, xb, wA);
-                if (mB != mA) dB[i] = make_z(xb, xa, wB);
+            float2 xa[2], xb[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                xa[u] = make_float2(4.f * accr[0][i + u][j], 4.f * acci[0][i + u][j]);
+                xb[u] = make_float2(4.f * accr[1][i + u][j], 4.f * acci[1][i + u][j]);
+                if (mp == 0) {              // X(0) and X(P) are real
+                    xa[u].y = 0.f;
+                    xb[u].y = 0.f;
+                }
+            }
+            const float2 a0 = make_z(xa[0], xb[0], wA), a1 = make_z(xa[1], xb[1], wA);
+            dA[i >> 1] = make_float4(a0.x, a1.x, a0.y, a1.y);
+            if (mp != 0 && mB != mA) {
+                const float2 b0 = make_z(xb[0], xa[0], wB), b1 = make_z(xb[1], xa[1], wB);
+                dB[i >> 1] = make_float4(b0.x, b1.x, b0.y, b1.y);
             }
         }
     }
@@ -639,11 +645,9 @@ __global__ void __launch_bounds__(256) k_stage1_fp32(int Ks, int P, const float2
 //            D(g + q P/Q) = Re sum_r i_Q^{q r} S_r (i_Q = exp(2 pi i/Q)); the twiddles
 //            w_P^{j g} come from an FP64 table in shared memory and are the same for the
 //            whole warp (broadcast reads).
-// Layouts of the stored factor: p2 == 0, natural Dinv[rl][col][rho] (P values); p2 > 0,
-// the order in which the split-radix stage 2 (P = P1 x p2) reads them, block pairs
-// (l2, l2 + 1) of its pass B: Dinv[rl][col][l2 >> 1][l1][b][l2 & 1] for
-// rot = 2 (l2 + p2 l1) + b (rho = rot mod P; for odd p2 lane 1 of the last pair repeats
-// l2 = p2 - 1; 4 P1 ceil(p2 / 2) values), multiplied by dscale.
+// The stored factor: natural, Dinv[rl][col][rho] (P values), for the general stage 2; for the
+// lengths with a fast stage 2 times dscale in the groups its pass B reads (S2Split in k_stage2.cu;
+// norm_slot below): one value for the two rotations rho and rho + P that share it.
 // FP32 copies of the normaliser's spectra, transposed so that the contraction below reads
 // them coalesced: RUf[j][k][r] = RU[r][j][k] (|ref|^2 spectra), CVf[j][k][c] = CV[c][j][k]
 // (CTF^2 spectra); the values the FP64 spectra round to, as the contraction always used
@@ -748,12 +752,10 @@ constexpr int NORM_RB = 32;
 constexpr int NORM_GPT = 3;
 template <int Q>
 __global__ void __launch_bounds__(256) k_norm(Geom g, const float2 *__restrict__ Yg, int nr, int c0, int ncols,
-                                              int dcols, const float *__restrict__ sqp, float *__restrict__ D, int p2,
-                                              double dscale)
+                                              int dcols, const float *__restrict__ sqp, float *__restrict__ D)
 {
     extern __shared__ double2 sd[];
     const int P = g.P, J = P / 2 + 1, G = P / Q, Jp = J | 1;
-    const int p1 = p2 > 0 ? P / p2 : 0, dlen = p2 > 0 ? 4 * p1 * ((p2 + 1) / 2) : P;
     double2 *Y = sd;                            // [NORM_RB][Jp], scaled by wgt_j / P
     double2 *tw = Y + (size_t)NORM_RB * Jp;     // [P] w_P^{+e}
     const int cl = blockIdx.x;
@@ -778,7 +780,7 @@ __global__ void __launch_bounds__(256) k_norm(Geom g, const float2 *__restrict__
         __syncthreads();
         if (lane < nb) {
             const double2 *y = Y + (size_t)lane * Jp;
-            float *dst = D + ((size_t)(rb0 + lane) * dcols + cl) * dlen;
+            float *dst = D + ((size_t)(rb0 + lane) * dcols + cl) * P;
             for (int g0 = warp * NORM_GPT; g0 < G; g0 += nwarps * NORM_GPT) {
                 double sr[NORM_GPT][Q], si[NORM_GPT][Q];
                 int idx[NORM_GPT];
@@ -821,19 +823,7 @@ __global__ void __launch_bounds__(256) k_norm(Geom g, const float2 *__restrict__
                             else if (4 * e == Q) d -= si[t][r];
                             else d += si[t][r];            // 4 e == 3 Q
                         }
-                        const int rho = gg + q * G;
-                        if (p2 == 0) {
-                            dst[rho] = (float)(1.0 / sqrt(d * sq));
-                        } else {
-                            const float v = (float)(dscale / sqrt(d * sq));
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {   // rot = rho and rho + P
-                                const int rot = rho + h * P, l = rot >> 1, l2 = l % p2;
-                                float *o = dst + ((((l2 >> 1) * p1 + l / p2) * 2 + (rot & 1)) * 2 + (l2 & 1));
-                                o[0] = v;
-                                if ((p2 & 1) && l2 == p2 - 1) o[1] = v;
-                            }
-                        }
+                        dst[gg + q * G] = (float)(1.0 / sqrt(d * sq));
                     }
                 }
             }
@@ -852,15 +842,21 @@ __global__ void __launch_bounds__(256) k_norm(Geom g, const float2 *__restrict__
 //   pass 1, task (reference, n1): a length-N2 DFT over n2 of conj Zh(n1 + N1 n2), times
 //           w_{P/2}^{-n1 k2}, into buf[reference][k2][n1];
 //   pass 2, task (reference, k2): a length-N1 DFT over n1 -> conj z(k2 + N2 k1).
-// P2C: the stage-2 split P = P1 x P2C the factors are laid out for (compile-time, so that the
-// layout's index arithmetic divides by a constant), or 0 for the natural layout
-template <int N1, int N2, int P2C>
+// The place of D(2l + b), l < P/2, in the groups of stage 2's split of P (S2Split)
+template <int P> __host__ __device__ constexpr int norm_dlen() { return P == 64 ? 64 : P == 180 ? 200 : 300; }
+template <int P> __device__ __forceinline__ int norm_slot(int l, int b)
+{
+    if (P == 64) return (l % 8) * 8 + (l / 8) * 2 + b;            // block l mod 8, l1 = l / 8 < 4
+    if (P == 180) return (l % 10) * 20 + (l % 9) * 2 + b;         // blocks l2 = l mod 20 and l2 + 10, l1 = l mod 9
+    return (l % 25) * 12 + (l % 6) * 2 + b;                       // P = 300: block l mod 25, l1 = l mod 12 and l1 + 6
+}
+
+template <int N1, int N2>
 __global__ void __launch_bounds__(256) k_norm_fft(const float2 *__restrict__ Yg, int nr, int c0, int ncols, int dcols,
                                                   const float *__restrict__ sqp, float *__restrict__ D, double dscale,
                                                   int eu)
 {
     constexpr int H = N1 * N2, P = 2 * H, J = H + 1;
-    constexpr int p2 = P2C;
     constexpr int NB = 256 / (N1 > N2 ? N1 : N2);
     extern __shared__ double2 sd[];
     double2 *tw = sd;                 // [H] w_{P/2}^{-e}
@@ -878,7 +874,7 @@ __global__ void __launch_bounds__(256) k_norm_fft(const float2 *__restrict__ Yg,
         wp[e] = make_double2(cs, sn);
     }
     const double sq = (double)sqp[col];
-    constexpr int p1 = p2 > 0 ? P / p2 : 0, dlen = p2 > 0 ? 4 * p1 * ((p2 + 1) / 2) : P;
+    constexpr int dlen = norm_dlen<P>();
     // a batch's Y rows (J values each, coalesced) by asynchronous 8-byte copies: the first batch's
     // before the loop, every later batch's while the previous batch's pass 2 runs (pass 1 has
     // consumed ys by then)
@@ -940,57 +936,36 @@ __global__ void __launch_bounds__(256) k_norm_fft(const float2 *__restrict__ Yg,
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const double d = b == 0 ? x[k1].x : -x[k1].y;   // D(2l + b)
-                    const int rho = 2 * l + b;
                     // the FP32 factor 1/sqrt(D sqsum): D sqsum formed in FP64, its reciprocal square
                     // root in FP32 by rsqrtf and one Newton-Raphson step y (3 - a y^2) / 2
                     const float a = (float)(d * sq);
                     float y = rsqrtf(a);
                     y = y * fmaf(-0.5f * a, y * y, 1.5f);
-                    if constexpr (p2 == 0) {
-                        dst[rho] = y;
-                    } else {
-                        // the Euclidean objective: the additive term -(D + sum_k w_k |ptcl_k|^2) / 2,
-                        // sq holding the weighted particle term
-                        const float v = eu ? (float)(-0.5 * (d + sq)) : (float)dscale * y;
-#pragma unroll
-                        for (int hh = 0; hh < 2; ++hh) {   // rot = rho and rho + P
-                            const int rot = rho + hh * P, lr = rot >> 1, l2 = lr % p2;
-                            float *o = dst + ((((l2 >> 1) * p1 + lr / p2) * 2 + (rot & 1)) * 2 + (l2 & 1));
-                            o[0] = v;
-                            if ((p2 & 1) && l2 == p2 - 1) o[1] = v;
-                        }
-                    }
+                    // the Euclidean objective: the additive term -(D + sum_k w_k |ptcl_k|^2) / 2,
+                    // sq holding the weighted particle term
+                    dst[norm_slot<P>(l, b)] = eu ? (float)(-0.5 * (d + sq)) : (float)dscale * y;
                 }
             }
         }
     }
 }
 
-template <int N1, int N2, int P2C>
-static cudaError_t launch_norm_fft_k(pftcc_handle *h, const float2 *Y, int nr, int c0, int ncols, int dcols,
-                                     const float *sqp, float *D, double dscale, int eu)
+template <int N1, int N2>
+static cudaError_t launch_norm_fft(pftcc_handle *h, const float2 *Y, int nr, int c0, int ncols, int dcols,
+                                   const float *sqp, float *D, double dscale, int eu)
 {
     constexpr int H = N1 * N2, NB = 256 / (N1 > N2 ? N1 : N2);
+    if (stage2_fast_dlen(2 * H) != norm_dlen<2 * H>()) return cudaErrorInvalidValue;
     const size_t smem = (size_t)(2 * H + NB * N2 * (N1 + 1)) * sizeof(double2) + (size_t)NB * (H + 1) * sizeof(float2);
-    cudaError_t e = smem_limit((const void *)k_norm_fft<N1, N2, P2C>, smem);
+    cudaError_t e = smem_limit((const void *)k_norm_fft<N1, N2>, smem);
     if (e != cudaSuccess) return e;
-    k_norm_fft<N1, N2, P2C><<<ncols, 256, smem, h->stream>>>(Y, nr, c0, ncols, dcols, sqp, D, dscale, eu);
+    k_norm_fft<N1, N2><<<ncols, 256, smem, h->stream>>>(Y, nr, c0, ncols, dcols, sqp, D, dscale, eu);
     return cudaGetLastError();
-}
-
-// the natural layout (p2 == 0) or the stage-2 split of the length (the only split served)
-template <int N1, int N2, int P2F>
-static cudaError_t launch_norm_fft(pftcc_handle *h, const float2 *Y, int nr, int c0, int ncols, int dcols,
-                                   const float *sqp, float *D, int p2, double dscale, int eu)
-{
-    if (p2 == 0) return launch_norm_fft_k<N1, N2, 0>(h, Y, nr, c0, ncols, dcols, sqp, D, dscale, eu);
-    if (p2 == P2F) return launch_norm_fft_k<N1, N2, P2F>(h, Y, nr, c0, ncols, dcols, sqp, D, dscale, eu);
-    return cudaErrorInvalidValue;
 }
 
 static cudaError_t launch_norm(pftcc_handle *h, const Geom &g, const float2 *RUf, int nrefs_p, const float2 *CVf,
                                int cols_pad, int r0, int nr, int c0, int ncols, int dcols, const float *sqp, float2 *Y,
-                               float *D, int p2, double dscale, int eu)
+                               float *D, double dscale, int eu)
 {
     const int J = g.P / 2 + 1;
     cudaError_t e;
@@ -1005,22 +980,22 @@ static cudaError_t launch_norm(pftcc_handle *h, const Geom &g, const float2 *RUf
     }
     PFTCC_LAUNCH(h);
     switch (g.P) {
-    case 64: return launch_norm_fft<8, 4, 8>(h, Y, nr, c0, ncols, dcols, sqp, D, p2, dscale, eu);
-    case 180: return launch_norm_fft<10, 9, 15>(h, Y, nr, c0, ncols, dcols, sqp, D, p2, dscale, eu);
-    case 300: return launch_norm_fft<15, 10, 20>(h, Y, nr, c0, ncols, dcols, sqp, D, p2, dscale, eu);
+    case 64: return launch_norm_fft<8, 4>(h, Y, nr, c0, ncols, dcols, sqp, D, dscale, eu);
+    case 180: return launch_norm_fft<10, 9>(h, Y, nr, c0, ncols, dcols, sqp, D, dscale, eu);
+    case 300: return launch_norm_fft<15, 10>(h, Y, nr, c0, ncols, dcols, sqp, D, dscale, eu);
     default: break;
     }
     if (eu) return cudaErrorInvalidValue;   // the Euclidean objective needs the transform lengths above
     const size_t smem = ((size_t)NORM_RB * (J | 1) + g.P) * sizeof(double2);
     if (g.P % 4 == 0) {
         if ((e = smem_limit((const void *)k_norm<4>, smem))) return e;
-        k_norm<4><<<ncols, 256, smem, h->stream>>>(g, Y, nr, c0, ncols, dcols, sqp, D, p2, dscale);
+        k_norm<4><<<ncols, 256, smem, h->stream>>>(g, Y, nr, c0, ncols, dcols, sqp, D);
     } else if (g.P % 2 == 0) {
         if ((e = smem_limit((const void *)k_norm<2>, smem))) return e;
-        k_norm<2><<<ncols, 256, smem, h->stream>>>(g, Y, nr, c0, ncols, dcols, sqp, D, p2, dscale);
+        k_norm<2><<<ncols, 256, smem, h->stream>>>(g, Y, nr, c0, ncols, dcols, sqp, D);
     } else {
         if ((e = smem_limit((const void *)k_norm<1>, smem))) return e;
-        k_norm<1><<<ncols, 256, smem, h->stream>>>(g, Y, nr, c0, ncols, dcols, sqp, D, p2, dscale);
+        k_norm<1><<<ncols, 256, smem, h->stream>>>(g, Y, nr, c0, ncols, dcols, sqp, D);
     }
     return cudaGetLastError();
 }
@@ -1068,12 +1043,15 @@ __global__ void k_stage2(S2Params sp, const float2 *__restrict__ X, const float 
     }
     __syncthreads();
     const size_t plane = (size_t)sp.xcols * sp.xrows;
-    const float2 *Xc = X + (size_t)cl * sp.xrows;
+    const float *Xc = reinterpret_cast<const float *>(X + (size_t)cl * sp.xrows);   // row pairs of (re, re, im, im)
     // X carries the factor 4 of the half-circle transforms; y/(2N) is the correlation sum
     const float scale = 1.0f / (2.0f * (float)N);
     for (int row = t; row < sp.rows; row += T) {
         // the packed spectrum Z as stage 1 stored it, digit-reversed into the slab
-        for (int j = 0; j < P; ++j) buf[(size_t)rev[j] * T + t] = Xc[(size_t)j * plane + row];
+        for (int j = 0; j < P; ++j) {
+            const float *v = Xc + 2 * ((size_t)j * plane + (row & ~1)) + (row & 1);
+            buf[(size_t)rev[j] * T + t] = make_float2(v[0], v[2]);
+        }
         // in-place mixed-radix DIT passes, innermost radix first
         int span = 1;   // m_l of the current level
         for (int l = sp.nf - 1; l >= 0; --l) {
@@ -1329,7 +1307,7 @@ int search_mdomain(pftcc_handle *h, int nshifts_in, const float *shifts_host, in
             (st = ensure_ws(h, (void **)&ws.UB, (size_t)M * cols_pad * Ks * sizeof(float2), "UB")) ||
             (st = ensure_ws(h, (void **)&ws.RU, (size_t)h->nrefs * J * Ks * sizeof(double2), "RU")) ||
             (st = ensure_ws(h, (void **)&ws.CV, (size_t)cols_pad * J * Ks * sizeof(double2), "CV")) ||
-            (st = ensure_ws(h, (void **)&ws.D, (size_t)nr_wave_max * W_cols * std::max(2 * P, stage2_fast_dlen(P)) * sizeof(float), "D")) ||
+            (st = ensure_ws(h, (void **)&ws.D, (size_t)nr_wave_max * W_cols * std::max(P, stage2_fast_dlen(P)) * sizeof(float), "D")) ||
             (st = ensure_ws(h, (void **)&ws.RUf, (size_t)h->nrefs * J * Ks * sizeof(float2), "RUf")) ||
             (st = ensure_ws(h, (void **)&ws.CVf, (size_t)cols_pad * J * Ks * sizeof(float2), "CVf")) ||
             (st = ensure_ws(h, (void **)&ws.Yn, (size_t)nr_wave_max * W_cols * J * sizeof(float2), "Y")) ||
@@ -1419,16 +1397,15 @@ int search_mdomain(pftcc_handle *h, int nshifts_in, const float *shifts_host, in
                     PFTCC_LAUNCH(h);
                     KTimer kt(h, PFTCC_K_STAGE1);
                     k_stage1_fp32<<<grid, 256, smem_s1, h->stream>>>(Ks, P, ws.UA, rows_pad, row0, ws.UB, cols_pad, c0,
-                                                                    ws.X, rows_t, cols_t);
+                                                                    reinterpret_cast<float4 *>(ws.X), rows_t, cols_t);
                     CKE(cudaGetLastError(), "stage1");
                 }
                 // the split-radix stage 2 reads the factor in its visiting order, times 1/(2N)
                 CKE(launch_norm(h, g, ws.RUf, h->nrefs, ws.CVf, cols_pad, r_lo, r_hi - r_lo + 1, c0, cols, cols_t,
-                                ws.sqp, ws.Yn, ws.D,
-                                fast_s2 ? stage2_fast_p2(P) : 0, 1.0 / (2.0 * N), eu), "norm");
+                                ws.sqp, ws.Yn, ws.D, 1.0 / (2.0 * N), eu), "norm");
                 if (fast_s2) {
                     e = launch_stage2_fast(h, P, rows, rows_t, cols_t, row0, ns, r_lo, cols_t, c0, cols, nrs, ws.X, ws.D,
-                                           ws.cand, ccall_dev, d_perm, eu);
+                                           ws.cand, ccall_dev, d_perm, eu, ntop == 0);
                     if (e != cudaSuccess)
                         return set_err(h, e == cudaErrorMemoryAllocation ? PFTCC_ERR_OOM : PFTCC_ERR_CUDA,
                                        "stage2 (P " + std::to_string(P) + ", rows " + std::to_string(rows) + ", columns " +
@@ -1482,7 +1459,7 @@ int search_mdomain(pftcc_handle *h, int nshifts_in, const float *shifts_host, in
 namespace pftcc {
 
 cudaError_t launch_stage2_waves(pftcc_handle *h, int P, std::vector<S2Wave> &waves, int nshifts, int nrs_total,
-                                float2 *cand, float *ccall, const int *perm, int eu);
+                                float2 *cand, float *ccall, const int *perm, int eu, int rot);
 
 // every held particle's best out of a searched group starts as "not searched" (reference 0)
 __global__ void k_best_clear(pftcc_best *out, int n)
@@ -1627,7 +1604,7 @@ int search_mdomain_groups(pftcc_handle *h, int ngroups, const int *ref0, const i
     const float *ctf = (h->cfg.with_ctf && h->ctf_ready) ? h->ctfmats : nullptr;
     const size_t smem_s1 = 4 * (size_t)Ks * S1_TILE * sizeof(float2);
     CKG(smem_limit((const void *)k_stage1_fp32, smem_s1), "attr");
-    const int p2 = stage2_fast_p2(P), dlen = stage2_fast_dlen(P);
+    const int dlen = stage2_fast_dlen(P);
     const bool md_rescore = ntop > 0 && h->cfg.ctf_frame == PFTCC_FRAME_PTCL;
     {
         const int st = umma_reset(h);    // the device error word of the bounded waits (allocated once)
@@ -1691,7 +1668,7 @@ int search_mdomain_groups(pftcc_handle *h, int ngroups, const int *ref0, const i
                 const WavePlan &p = plan[w1];
                 const size_t z = (size_t)P * (p.a_hi - p.a_lo) * (p.t_hi - p.t_lo) * COL_TILE * sizeof(float2);
                 const int nrw = (p.r_hi - 1) / ns - p.r_lo / ns + 1;
-                const size_t d = (size_t)nrw * (p.c_hi - p.c_lo) * std::max(2 * P, dlen) * sizeof(float);
+                const size_t d = (size_t)nrw * (p.c_hi - p.c_lo) * dlen * sizeof(float);
                 const size_t y = (size_t)nrw * (p.c_hi - p.c_lo) * J * sizeof(float2);
                 if (w1 > w0 && (zb + z > z_batch_max || db + d > d_batch_max)) break;
                 zb += z; db += d; yb = std::max(yb, y); ++w1;
@@ -1719,21 +1696,21 @@ int search_mdomain_groups(pftcc_handle *h, int ngroups, const int *ref0, const i
                     PFTCC_LAUNCH(h);
                     KTimer kt(h, PFTCC_K_STAGE1);
                     k_stage1_fp32<<<grid, 256, smem_s1, h->stream>>>(Ks, P, ws.UA, rows_pad, p.a_lo, ws.UB, cols_pad,
-                                                                    p.t_lo * COL_TILE, Xw, xrows, xcols);
+                                                                    p.t_lo * COL_TILE, reinterpret_cast<float4 *>(Xw), xrows, xcols);
                     CKG(cudaGetLastError(), "stage1");
                 }
                 CKG(launch_norm(h, g, ws.RUf, h->nrefs, ws.CVf, cols_pad, r_lo_ref, nrw, p.c_lo, cols, cols, ws.sqp,
-                                ws.Yn, Dw, p2, 1.0 / (2.0 * N), 0), "norm");
+                                ws.Yn, Dw, 1.0 / (2.0 * N), 0), "norm");
                 s2.push_back(S2Wave{Xw, Dw, p.r_lo, p.r_hi - p.r_lo, p.r_lo - p.a_lo, xrows, xcols, p.c_lo, cols,
                                     p.c_lo - p.t_lo * COL_TILE, r_lo_ref, cols, 0, 0});
                 zo += (size_t)P * xrows * xcols * sizeof(float2);
-                dof += (size_t)nrw * cols * std::max(2 * P, dlen) * sizeof(float);
+                dof += (size_t)nrw * cols * dlen * sizeof(float);
             }
             if (precision == PFTCC_PREC_BF16X3) {
                 st = umma_stage1_waves(h, M, s1);
                 if (st != PFTCC_OK) return st;
             }
-            e = launch_stage2_waves(h, P, s2, ns, nrs, ws.cand, nullptr, bperm, 0);
+            e = launch_stage2_waves(h, P, s2, ns, nrs, ws.cand, nullptr, bperm, 0, ntop == 0);
             if (e != cudaSuccess)
                 return set_err(h, e == cudaErrorMemoryAllocation ? PFTCC_ERR_OOM : PFTCC_ERR_CUDA,
                                std::string("grouped stage 2: ") + cudaGetErrorString(e));

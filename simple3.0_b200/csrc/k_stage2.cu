@@ -13,8 +13,8 @@
 //   pass A: for each residue class j1 < P1 a length-P2 DFT over j2 of Z(j1 + P1 j2),
 //           times w_P^{-j1 l2}, into a thread-private shared-memory slab;
 //   pass B: for each l2 < P2 a length-P1 DFT over j1 -> z(l2 + P2 l1).
-// The search (k_stage2_fast) reads Z as stage 1 stored it, P planes of [col][row]; the
-// FP32 re-score forms Z from X itself, processing classes j1 and P1 - j1 together so
+// The search (k_stage2_fast; S2Split gives its splits) reads Z as stage 1 stored it, P planes of
+// [col][row pair] (re, re, im, im); the FP32 re-score forms Z from X itself, processing classes j1 and P1 - j1 together so
 // that every X element is computed once (Z(j) needs X(j) and X(P - j), which lie in the
 // mirror class).
 #include "pftcc_internal.cuh"
@@ -242,61 +242,6 @@ template <int STEP> struct PFFT<1, STEP> {
     __device__ static void run(C2 *, const TwTables &) {}
 };
 
-// Row slab of the search (two-lane layout): pass-A output (l2, j1) -- re and im as two
-// scalars -- sits in lane l2 & 1 of the float2 slots ((l2 >> 1) P1 + j1) 2 + part
-// (part 0 = re, 1 = im), element stride T, so that pass B reads the pair of blocks
-// (l2, l2 + 1) with one 8-byte load per part.  For odd P2 the last block l2 = P2 - 1 is
-// stored in both lanes.
-
-// the loads of class pair (c, cb) of one row: Z(c + P1 j2) and Z(cb + P1 j2)
-template <int P1, int P2, class GetZ>
-__device__ __forceinline__ void load_pair(int c, int cb, const GetZ &getz, float2 (&na)[P2], float2 (&nb)[P2])
-{
-#pragma unroll
-    for (int j2 = 0; j2 < P2; ++j2) {
-        na[j2] = getz(c + P1 * j2);
-        nb[j2] = getz(cb + P1 * j2);
-    }
-}
-
-// pass A of the search over the packed spectrum Z, two classes per step: c and cb = c + 1
-// (c again for the last class of an odd range), one per lane -- a length-P2 DFT over j2
-// of Z(c + P1 j2), times w_P^{-c l2} (lane-pair twiddles twa / twb, entry c P2 + l2), into
-// the slab.  na / nb hold the first pair's loads on entry (issued by the caller during the
-// previous row's pass B); the next pair's 2 P2 loads are issued before each transform.
-template <int P1, int P2, class GetZ>
-__device__ __forceinline__ void passA_pk(int c0, int c1, const GetZ &getz, float2 *slab, int T, const float4 *twa,
-                                         const float2 *twb, const TwTables &tw, float2 (&na)[P2], float2 (&nb)[P2])
-{
-#pragma unroll 1
-    for (int c = c0; c < c1; c += 2) {
-        const int cb = min(c + 1, c1 - 1);
-        C2 z[P2];
-#pragma unroll
-        for (int j2 = 0; j2 < P2; ++j2) z[j2] = {make_float2(na[j2].x, nb[j2].x), make_float2(na[j2].y, nb[j2].y)};
-        if (c + 2 < c1) load_pair<P1, P2>(c + 2, min(c + 3, c1 - 1), getz, na, nb);
-        PFFT<P2, P1>::run(z, tw);
-        float2 *sa = slab + (size_t)c * 2 * T, *sb = slab + (size_t)cb * 2 * T;
-#pragma unroll
-        for (int l2 = 0; l2 < P2; ++l2) {
-            C2 o = z[l2];
-            if (l2 > 0) {
-                const float4 w = twa[c * P2 + l2];
-                o = p_twid(o, make_float2(w.x, w.y), make_float2(w.z, w.w), twb[c * P2 + l2]);
-            }
-            const int q = (l2 >> 1) * P1 * 2;
-#pragma unroll
-            for (int ln = 0; ln < 2; ++ln) {
-                if (ln != (l2 & 1) && !((P2 & 1) && l2 == P2 - 1)) continue;
-                reinterpret_cast<float *>(sa + q * T)[ln] = o.r.x;
-                reinterpret_cast<float *>(sa + (q + 1) * T)[ln] = o.i.x;
-                reinterpret_cast<float *>(sb + q * T)[ln] = o.r.y;
-                reinterpret_cast<float *>(sb + (q + 1) * T)[ln] = o.i.y;
-            }
-        }
-    }
-}
-
 // Pass A, split into the pieces the two halves of a row's transform take: class 0 (its
 // own mirror, X(P) closes it), the class pairs (c, P1 - c) for C0 <= c < C1, and for even
 // P1 the self-mirrored class P1/2.  Outputs, times w_P^{-j1 l2}, go to the row's slab
@@ -395,119 +340,6 @@ __device__ __forceinline__ void passB(int L0, int L1, const float2 *slab, int T,
     }
 }
 
-// pass B on the block pair (l, l + 1), l even: two length-P1 DFTs (one per lane) of the
-// slab blocks, times the normalising factors -- stored in pair order, four per l1:
-// (l, re), (l + 1, re), (l, im), (l + 1, im), already carrying the 1/(2N) scale -- leaving
-// the correlation of rot = 2 (l + lane + P2 l1) + part in lane `lane` of v[l1].r / v[l1].i.
-// EU: the factors are the Euclidean objective's additive terms, the value escale * v + d
-template <int P1, int P2, bool EU>
-__device__ __forceinline__ void passB_pair(int l, const float2 *slab, int T, const TwTables &tw, const float4 *Dp,
-                                           float escale, C2 (&v)[P1])
-{
-    const float4 *dq = Dp + (size_t)(l >> 1) * P1;
-    float4 d[P1];
-#pragma unroll
-    for (int l1 = 0; l1 < P1; ++l1) d[l1] = __ldg(dq + l1);   // issued ahead of the transform
-    const float2 *sq = slab + (size_t)(l >> 1) * P1 * 2 * T;
-#pragma unroll
-    for (int j1 = 0; j1 < P1; ++j1) v[j1] = {sq[(2 * j1) * T], sq[(2 * j1 + 1) * T]};
-    PFFT<P1, P2>::run(v, tw);
-    if constexpr (EU) {
-        const float2 sc = f2_s(escale);
-#pragma unroll
-        for (int l1 = 0; l1 < P1; ++l1) {
-            v[l1].r = f2_fma(v[l1].r, sc, make_float2(d[l1].x, d[l1].y));
-            v[l1].i = f2_fma(v[l1].i, sc, make_float2(d[l1].z, d[l1].w));
-        }
-    } else {
-#pragma unroll
-        for (int l1 = 0; l1 < P1; ++l1) {
-            v[l1].r = f2_mul(v[l1].r, make_float2(d[l1].x, d[l1].y));
-            v[l1].i = f2_mul(v[l1].i, make_float2(d[l1].z, d[l1].w));
-        }
-    }
-}
-
-// pass B of the search for the block pairs (l, l + 1), l = L0, L0 + 2, ... < L1 (L0 even;
-// for odd P2 the pair (P2 - 1, P2) holds block P2 - 1 twice): the maximum correlation and
-// its rotation (lowest rotation among equal maxima).  Each pair's 4 P1 values are reduced
-// with max; afterwards the winning pair -- every pair when another one reached the same
-// maximum -- is evaluated again by the same code (identical values) and scanned for the
-// lowest rotation holding the maximum.
-template <int P1, int P2, bool EU>
-__device__ __forceinline__ void passB_search(int L0, int L1, const float2 *slab, int T, const TwTables &tw,
-                                             const float4 *Dp, float escale, float &best, int &brot)
-{
-    float bv = -INFINITY;
-    int bl = -1, l = L0, lend = L1, stage = 0, rmin = 0x7fffffff;
-    bool tie = false;
-#pragma unroll 1
-    while (true) {
-        C2 v[P1];
-        passB_pair<P1, P2, EU>(l, slab, T, tw, Dp, escale, v);
-        if (stage == 0) {
-            float m = fmaxf(v[0].r.x, v[0].r.y);
-            m = max3f(m, v[0].i.x, v[0].i.y);
-#pragma unroll
-            for (int l1 = 1; l1 < P1; ++l1) {
-                m = max3f(m, v[l1].r.x, v[l1].r.y);
-                m = max3f(m, v[l1].i.x, v[l1].i.y);
-            }
-            if (m > bv) { bv = m; bl = l; tie = false; }
-            else if (m == bv) tie = true;
-            l += 2;
-            if (l < L1) continue;
-            if (bl < 0) break;
-            stage = 1;
-            l = tie ? L0 : bl;
-            lend = tie ? L1 : bl + 2;
-        } else {
-            const int lb = min(l + 1, P2 - 1);
-#pragma unroll
-            for (int l1 = 0; l1 < P1; ++l1) {
-                const int ra = 2 * (l + P2 * l1), rb = 2 * (lb + P2 * l1);
-                if (v[l1].r.x == bv) rmin = min(rmin, ra);
-                if (v[l1].i.x == bv) rmin = min(rmin, ra + 1);
-                if (v[l1].r.y == bv) rmin = min(rmin, rb);
-                if (v[l1].i.y == bv) rmin = min(rmin, rb + 1);
-            }
-            l += 2;
-            if (l >= lend) break;
-        }
-    }
-    best = bv;
-    brot = bl < 0 ? 0 : rmin;
-}
-
-// pass B writing every correlation (corr_all), with the per-rotation argmax
-template <int P1, int P2, bool EU>
-__device__ __forceinline__ void passB_all(int L0, int L1, const float2 *slab, int T, const TwTables &tw,
-                                          const float4 *Dp, float escale, float *cc_out, float &best, int &brot)
-{
-#pragma unroll 1
-    for (int l = L0; l < L1; l += 2) {
-        C2 v[P1];
-        passB_pair<P1, P2, EU>(l, slab, T, tw, Dp, escale, v);
-        const bool two = l + 1 < P2;
-#pragma unroll
-        for (int l1 = 0; l1 < P1; ++l1) {
-            const float cv[4] = {v[l1].r.x, v[l1].i.x, v[l1].r.y, v[l1].i.y};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (e >= 2 && !two) continue;
-                const int r = 2 * (l + (e >> 1) + P2 * l1) + (e & 1);
-                cc_out[r] = cv[e];
-                if (cv[e] > best || (cv[e] == best && r < brot)) { best = cv[e]; brot = r; }
-            }
-        }
-    }
-}
-
-// how a row's transform is split between its NT threads: thread (role) r takes the class
-// pairs [r n / NT, (r + 1) n / NT) of the n = ceil(P1 / 2) pairs (2k, 2k + 1) of pass A and the
-// block pairs likewise of the ceil(P2 / 2) pairs (2q, 2q + 1) of pass B
-__host__ __device__ constexpr int role_part(int n, int r, int nt) { return r * n / nt; }
-
 // the whole per-triple transform in one thread; getx(j) returns X(j) for j = 0..P;
 // dinv(rot) the normalising factor; slab is this thread's shared-memory slab with
 // element stride T
@@ -527,28 +359,64 @@ struct S2Fast {
     float escale;   // the Euclidean objective: the transform's scale 1/(2N) (the factors are additive)
 };
 
-// the normalising factors per (reference, particle) in the order the search's pass B
-// reads them: 4 P1 values per block pair, ceil(P2 / 2) pairs (the last pair of an odd P2
-// repeats block P2 - 1)
-template <int P1, int P2> __host__ __device__ constexpr int s2_dlen() { return 4 * P1 * ((P2 + 1) / 2); }
-
-// threads per row of the search's stage 2
-constexpr int S2_THREADS_PER_ROW = 2;
-
 // (c, id) ranks above (c2, id2): larger correlation, then lower id
 __device__ __forceinline__ bool ranks_above(float c, int id, float c2, int id2) { return c > c2 || (c == c2 && id < id2); }
 
-// ROWS rows in flight per block, NT threads per row: warps w + r ROWS/32 (role r) share the
-// rows' slabs and meet at named barrier 1 + w twice per row (after pass A; after pass B, when
-// roles 1.. hand their argmax over).  Role 0 keeps its rows' running top-8 in registers; at
-// the end the block merges those lists with the particle's running top-8.
-// X here is the packed spectrum Z, P planes of [col][row].
-template <int P1, int P2, int ROWS, int NT, bool WRITE, bool EU>
-__global__ void __launch_bounds__(NT * ROWS, 1) k_stage2_fast(S2Fast sp, const TwTables tw, const S2Wave *__restrict__ waves,
-                                                            float2 *__restrict__ cand, float *__restrict__ ccall,
-                                                            const int *__restrict__ perm)
+// The search's split P = P1 x P2: pass A takes the P1 classes, a length-P2 DFT each, pass B the P2
+// blocks, a length-P1 DFT each, one class or block at a time per role (warp) of a row group.
+//   coprime factors (180 = 9 x 20, 300 = 12 x 25): the Good-Thomas mapping, class c holding the
+//     inputs j = P2 c + P1 j2 (mod P) and block l2 giving the outputs l = l1 (mod P1) = l2 (mod P2):
+//     no twiddles between the passes;
+//   64 = 8 x 8: class c holds j = c + P1 j2, twiddles w_P^{-c l2}, block l2 the outputs l2 + P2 l1.
+// Rotations 2l + b and 2l + b + P share their normalising factor, that is outputs l and l + P/2:
+// at P = 180 blocks l2 and l2 + 10 (the same l1), at 64 and 300 the outputs l1 and l1 + P1/2 of a
+// block.  A factor group q is the block(s) that use one set of DV factors, DQ its stride in memory
+// (a multiple of four, for 16-byte loads): factor (l1, b) of group q at q DQ + 2 l1 + b.
+// ROLES warps share 32 row pairs; MB blocks per SM.
+template <int P> struct S2Split;
+template <> struct S2Split<64> { static constexpr int P1 = 8, P2 = 8, PFA = 0, NQ = 8, BPQ = 1, DV = 8, DQ = 8, ROLES = 8, MB = 4; };
+template <> struct S2Split<180> { static constexpr int P1 = 9, P2 = 20, PFA = 1, NQ = 10, BPQ = 2, DV = 18, DQ = 20, ROLES = 10, MB = 2; };
+template <> struct S2Split<300> { static constexpr int P1 = 12, P2 = 25, PFA = 1, NQ = 25, BPQ = 1, DV = 12, DQ = 12, ROLES = 13, MB = 1; };
+
+// the normalising factors of the length: floats per (reference, particle)
+template <int P> __host__ __device__ constexpr int s2_dlen() { return S2Split<P>::NQ * S2Split<P>::DQ; }
+
+// output index l of block l2 at l1
+template <int P> __device__ __forceinline__ int s2_out(int l1, int l2)
 {
-    constexpr int Q2 = (P2 + 1) / 2, DLEN = s2_dlen<P1, P2>(), NPA = (P1 + 1) / 2;
+    using S = S2Split<P>;
+    if constexpr (S::PFA) {
+        constexpr int E1 = crt_c(1, 0, S::P1, S::P2), E2 = crt_c(0, 1, S::P1, S::P2);   // 1 and 0 modulo (P1, P2), and 0 and 1
+        return (E1 * l1 + E2 * l2) % P;
+    } else {
+        return l2 + S::P2 * l1;
+    }
+}
+
+// What bounds it: the DRAM read of Z (1,440 B a triple at P = 180), with the transforms' FP32 pipe time
+// at half of that.  A block takes one particle column, 32 row pairs (64 rows) at a time: lane = row
+// pair, whose two rows go through the two lanes of the f32x2 instructions, so that a 16-byte load of Z
+// (stage 1 stores re, re, im, im of a row pair) is an operand as it comes, and warp = role.  Per
+// iteration: pass A from global memory into the slab [P2 blocks][P1][32 lanes] of 16 bytes, a barrier,
+// pass B from the slab to the maximum over the rotations, a barrier.  The small per-role state lets
+// 20 warps share an SM where one thread per class pair and row needed 254 registers and 8 warps; the
+// coprime splits have no twiddles, the row pairs no packing moves, and the factors are read once for
+// both rotations that share them.  Only what the caller uses is computed: with a re-score to follow
+// (ROT false) a candidate is its row, so the winning rotation is not searched for.
+// The last role keeps the block's running top 8 per lane in shared memory, fed a barrier later.
+// Measured, ms before (a column per block, two threads per row, 128 rows, class pairs in the lanes) and
+// now: 500 references x 81 shifts x 20,000 particles, P = 180: 395, 256 (4.6 TB/s of Z); 100 references
+// x 1000 particles, P = 64: 0.159, 0.028; 300 x 5130 pairs' groups, P = 300: 1.26, 0.59.  At P = 180,
+// 3.2e7 triples: 10 roles 9.5 ms (4.9 TB/s), 9 roles 10.5, 5 roles 10.0, 12 roles 13.2 (spills), the
+// next rows prefetched into L2 9.8; P = 300, 2.5e6 triples: 13 roles 1.65, 12 1.68, 9 2.05, 8 1.93;
+// P = 64, 5e6 triples: 8 roles x 4 blocks 0.56, x 3 0.64, x 5 0.72, 4 roles x 6 0.82.
+template <int P, bool ROT, bool WRITE, bool EU>
+__global__ void __launch_bounds__(32 * S2Split<P>::ROLES, S2Split<P>::MB)
+k_stage2_fast(S2Fast sp, const __grid_constant__ TwTables tw, const S2Wave *__restrict__ waves, float2 *__restrict__ cand,
+              float *__restrict__ ccall, const int *__restrict__ perm)
+{
+    using S = S2Split<P>;
+    constexpr int P1 = S::P1, P2 = S::P2, NR = S::ROLES, DLEN = s2_dlen<P>();
     // this block's wave (the last one starting at or before it) and column within it
     int lo = 0, hi = sp.nwaves - 1;
     while (lo < hi) {
@@ -557,137 +425,173 @@ __global__ void __launch_bounds__(NT * ROWS, 1) k_stage2_fast(S2Fast sp, const T
     }
     const S2Wave *W = waves + lo;
     const int cl = (int)blockIdx.x - __ldg(&W->blk0);
-    const float2 *X = reinterpret_cast<const float2 *>(__ldg(reinterpret_cast<const unsigned long long *>(&W->X)));
+    const float4 *X = reinterpret_cast<const float4 *>(__ldg(reinterpret_cast<const unsigned long long *>(&W->X)));
     const float *Dinv = reinterpret_cast<const float *>(__ldg(reinterpret_cast<const unsigned long long *>(&W->D)));
     const int w_rows = __ldg(&W->rows), w_row0 = __ldg(&W->row0), w_rofs = __ldg(&W->rofs);
     const int w_xrows = __ldg(&W->xrows), w_xcols = __ldg(&W->xcols), w_col0 = __ldg(&W->col0);
     const int w_zc0 = __ldg(&W->zc0), w_r0 = __ldg(&W->r0), w_dcols = __ldg(&W->dcols);
     extern __shared__ float4 smem4[];
-    const int t = threadIdx.x;
-    const int role = t / ROWS, lr = t - role * ROWS;
-    const int bar = 1 + (lr >> 5);
-    float2 *slab = reinterpret_cast<float2 *>(smem4) + lr;                                      // [Q2 P1 2][ROWS]
-    float4 *twa = smem4 + (size_t)Q2 * P1 * ROWS;                                               // [P1 P2]
-    float2 *twb = reinterpret_cast<float2 *>(twa + P1 * P2);                                    // [P1 P2]
-    float *xfer_c = reinterpret_cast<float *>(twb + P1 * P2);                                   // [NT - 1][ROWS]
-    int *xfer_r = reinterpret_cast<int *>(xfer_c + (NT - 1) * ROWS);                            // [NT - 1][ROWS]
-    // lane-pair twiddles of pass A: lane a class c, lane b class min(c + 1, P1 - 1) (pairs
-    // start at even classes in every role's range)
-    for (int e = t; e < P1 * P2; e += blockDim.x) {
-        const int c = e / P2, l2 = e - c * P2;
-        const int cb = min(c + 1, P1 - 1);
-        const float2 wa = tw.wP[c * l2], wb = tw.wP[cb * l2];
-        twa[e] = make_float4(wa.x, wb.x, wa.y, wb.y);
-        twb[e] = make_float2(-wa.y, -wb.y);
-    }
-    __syncthreads();
-    // Z offsets in float2 units fit 32 bits (the launcher checks P xcols xrows < 2^32); the wave's
-    // rows start at Z row w_rofs
-    const uint32_t plane = (uint32_t)w_xcols * (uint32_t)w_xrows;
-    const float2 *Xc = X + (size_t)(w_zc0 + cl) * w_xrows + w_rofs;
-    float kc[8];
-    int ki[8];
+    const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
+    float4 *slab = smem4 + lane;                                                  // [P2 P1][32]
+    float2 *xfer = reinterpret_cast<float2 *>(smem4 + P * 32);                    // [NR][32] the roles' maxima of the row pairs
+    int2 *xrot = reinterpret_cast<int2 *>(xfer + NR * 32);                        // [NR][32] their rotations (ROT)
+    float *kc = reinterpret_cast<float *>(xrot + (ROT ? NR * 32 : 0));            // [8][32] each lane's running top 8
+    int *ki = reinterpret_cast<int *>(kc + 8 * 32);
+    if (role == NR - 1)
+        for (int k = 0; k < 8; ++k) { kc[k * 32 + lane] = -INFINITY; ki[k * 32 + lane] = 0x7fffffff; }
+    // Z offsets in float4 units fit 32 bits (the launcher checks P xcols xrows < 2^32)
+    const uint32_t plane = (uint32_t)w_xcols * (uint32_t)(w_xrows >> 1);
+    const int pr0 = w_rofs >> 1, pr1 = (w_rofs + w_rows - 1) >> 1;                // the wave's row pairs of Z
+    const float4 *Xc = X + (size_t)(w_zc0 + cl) * (w_xrows >> 1);
+    const float *Dc = Dinv + (size_t)cl * DLEN;
+    auto merge = [&](int base) {   // the row pairs base + lane, after their pass B
+        const int r0 = 2 * (base + lane) - w_rofs;
+        float2 b = make_float2(-INFINITY, -INFINITY);
+        int2 br = make_int2(0, 0);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { kc[k] = -INFINITY; ki[k] = 0x7fffffff; }
-    // this role's classes [ca, ce) of Z and pass-B blocks [lb0, lb1)
-    const int ca = 2 * role_part(NPA, role, NT), ce = min(P1, 2 * role_part(NPA, role + 1, NT));
-    const int lb0 = 2 * role_part(Q2, role, NT), lb1 = min(P2, 2 * role_part(Q2, role + 1, NT));
-    auto zload = [&](int row) {
-        const float2 *xr = Xc + row;
-        return [=](int j) {
-            float2 v;
-            asm volatile("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];"
-                         : "=f"(v.x), "=f"(v.y)
-                         : "l"(xr + (uint32_t)j * plane));
-            return v;
-        };
-    };
-    float2 na[P2], nb[P2];   // the first class pair of this thread's next row
-    if (lr < w_rows && ca < ce) load_pair<P1, P2>(ca, min(ca + 1, ce - 1), zload(lr), na, nb);
-    for (int base = 0; base < w_rows; base += ROWS) {
-        const int row = base + lr;
-        const bool active = row < w_rows;
-        const int grow = w_row0 + row;
-        // this row's reference: its factors in pass-B order
-        const float4 *Dr = reinterpret_cast<const float4 *>(
-            Dinv + ((size_t)(grow / sp.nshifts - w_r0) * w_dcols + cl) * DLEN);
-        if (active) passA_pk<P1, P2>(ca, ce, zload(row), slab, ROWS, twa, twb, tw, na, nb);
-        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * NT) : "memory");
-        if (row + ROWS < w_rows && ca < ce) load_pair<P1, P2>(ca, min(ca + 1, ce - 1), zload(row + ROWS), na, nb);
-        float best = -INFINITY;
-        int brot = 0;
-        if (active) {
-            if constexpr (WRITE) {
-                float *cc_out = ccall + ((size_t)perm[w_col0 + cl] * sp.nrs_total + grow) * sp.N;
-                passB_all<P1, P2, EU>(lb0, lb1, slab, ROWS, tw, Dr, sp.escale, cc_out, best, brot);
+        for (int r = 0; r < NR; ++r) {
+            const float2 v = xfer[r * 32 + lane];
+            if constexpr (ROT) {
+                const int2 o = xrot[r * 32 + lane];
+                if (v.x > b.x || (v.x == b.x && o.x < br.x)) { b.x = v.x; br.x = o.x; }
+                if (v.y > b.y || (v.y == b.y && o.y < br.y)) { b.y = v.y; br.y = o.y; }
             } else {
-                passB_search<P1, P2, EU>(lb0, lb1, slab, ROWS, tw, Dr, sp.escale, best, brot);
+                b.x = fmaxf(b.x, v.x);
+                b.y = fmaxf(b.y, v.y);
             }
-            if (role > 0) { xfer_c[(role - 1) * ROWS + lr] = best; xfer_r[(role - 1) * ROWS + lr] = brot; }
         }
-        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * NT) : "memory");
-        if (active && role == 0) {
 #pragma unroll
-            for (int r = 1; r < NT; ++r) {
-                const float oc = xfer_c[(r - 1) * ROWS + lr];
-                const int orot = xfer_r[(r - 1) * ROWS + lr];
-                if (oc > best || (oc == best && orot < brot)) { best = oc; brot = orot; }
+        for (int i = 0; i < 2; ++i) {
+            float c = i ? b.y : b.x;
+            const int row = r0 + i;
+            if (row < 0 || row >= w_rows || c == -INFINITY || c < kc[7 * 32 + lane]) continue;
+            int id = (w_row0 + row) * sp.N + (ROT ? (i ? br.y : br.x) : 0);
+            for (int k = 0; k < 8; ++k) {
+                const float tc = kc[k * 32 + lane];
+                const int ti = ki[k * 32 + lane];
+                if (ranks_above(c, id, tc, ti)) { kc[k * 32 + lane] = c; ki[k * 32 + lane] = id; c = tc; id = ti; }
             }
-            if (best != -INFINITY) {
-                // insert into the running top-8 (kept sorted)
-                float c = best;
-                int id = grow * sp.N + brot;
+        }
+    };
+#pragma unroll 1
+    for (int base = pr0; base <= pr1; base += 32) {
+        const int pr = min(base + lane, pr1);   // lanes past the end repeat the last pair
+#pragma unroll 1
+        for (int c = role; c < P1; c += NR) {
+            const float4 *xr = Xc + pr;
+            C2 z[P2];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    if (ranks_above(c, id, kc[k], ki[k])) {
-                        const float tc = kc[k];
-                        const int ti = ki[k];
-                        kc[k] = c; ki[k] = id; c = tc; id = ti;
+            for (int j2 = 0; j2 < P2; ++j2) {
+                int j = S::PFA ? P2 * c + P1 * j2 : c + P1 * j2;
+                if (S::PFA && j >= P) j -= P;
+                asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(z[j2].r.x), "=f"(z[j2].r.y), "=f"(z[j2].i.x), "=f"(z[j2].i.y)
+                             : "l"(xr + (uint32_t)j * plane));
+            }
+            PFFT<P2, P1>::run(z, tw);
+#pragma unroll
+            for (int l2 = 0; l2 < P2; ++l2) {
+                C2 o = z[l2];
+                if (!S::PFA && l2 > 0) o = p_twid(o, tw.pc[c * l2], tw.ps[c * l2], tw.pn[c * l2]);
+                slab[(l2 * P1 + c) * 32] = make_float4(o.r.x, o.r.y, o.i.x, o.i.y);
+            }
+        }
+        if (role == NR - 1 && base > pr0) merge(base - 32);
+        __syncthreads();
+        const int row0 = min(max(2 * pr - w_rofs, 0), w_rows - 1), row1 = min(2 * pr + 1 - w_rofs, w_rows - 1);
+        const float *D0 = Dc + (size_t)((w_row0 + row0) / sp.nshifts - w_r0) * w_dcols * DLEN;
+        const float *D1 = Dc + (size_t)((w_row0 + row1) / sp.nshifts - w_r0) * w_dcols * DLEN;
+        float *cc0 = nullptr, *cc1 = nullptr;
+        if constexpr (WRITE) {
+            const int r0 = 2 * (base + lane) - w_rofs;
+            float *col = ccall + ((size_t)perm[w_col0 + cl] * sp.nrs_total + w_row0) * sp.N;
+            if (r0 >= 0 && r0 < w_rows) cc0 = col + (size_t)r0 * sp.N;
+            if (r0 + 1 < w_rows) cc1 = col + (size_t)(r0 + 1) * sp.N;
+        }
+        float2 best = make_float2(-INFINITY, -INFINITY);
+        int2 brot = make_int2(0x7fffffff, 0x7fffffff);
+#pragma unroll 1
+        for (int q = role; q < S::NQ; q += NR) {
+            float4 d0[S::DQ / 4], d1[S::DQ / 4];   // issued ahead of the transforms
+#pragma unroll
+            for (int e = 0; e < S::DQ / 4; ++e) {
+                d0[e] = __ldg(reinterpret_cast<const float4 *>(D0 + q * S::DQ) + e);
+                d1[e] = __ldg(reinterpret_cast<const float4 *>(D1 + q * S::DQ) + e);
+            }
+            const float *f0 = reinterpret_cast<const float *>(d0), *f1 = reinterpret_cast<const float *>(d1);
+#pragma unroll
+            for (int h = 0; h < S::BPQ; ++h) {
+                const int l2 = q + S::NQ * h;
+                C2 v[P1];
+#pragma unroll
+                for (int c = 0; c < P1; ++c) {
+                    const float4 a = slab[(l2 * P1 + c) * 32];
+                    v[c] = {make_float2(a.x, a.y), make_float2(a.z, a.w)};
+                }
+                PFFT<P1, P2>::run(v, tw);
+#pragma unroll
+                for (int l1 = 0; l1 < P1; ++l1) {
+                    constexpr int HALF = S::BPQ == 2 ? P1 : P1 / 2;
+                    const int e = 2 * (l1 % HALF);
+                    const float a0 = EU ? fmaf(v[l1].r.x, sp.escale, f0[e]) : v[l1].r.x * f0[e];
+                    const float a1 = EU ? fmaf(v[l1].i.x, sp.escale, f0[e + 1]) : v[l1].i.x * f0[e + 1];
+                    const float b0 = EU ? fmaf(v[l1].r.y, sp.escale, f1[e]) : v[l1].r.y * f1[e];
+                    const float b1 = EU ? fmaf(v[l1].i.y, sp.escale, f1[e + 1]) : v[l1].i.y * f1[e + 1];
+                    if constexpr (ROT) {
+                        const int rot = 2 * s2_out<P>(l1, l2);
+                        if (a0 > best.x || (a0 == best.x && rot < brot.x)) { best.x = a0; brot.x = rot; }
+                        if (a1 > best.x || (a1 == best.x && rot + 1 < brot.x)) { best.x = a1; brot.x = rot + 1; }
+                        if (b0 > best.y || (b0 == best.y && rot < brot.y)) { best.y = b0; brot.y = rot; }
+                        if (b1 > best.y || (b1 == best.y && rot + 1 < brot.y)) { best.y = b1; brot.y = rot + 1; }
+                        if constexpr (WRITE) {
+                            if (cc0) *reinterpret_cast<float2 *>(cc0 + rot) = make_float2(a0, a1);
+                            if (cc1) *reinterpret_cast<float2 *>(cc1 + rot) = make_float2(b0, b1);
+                        }
+                    } else {
+                        best.x = max3f(best.x, a0, a1);
+                        best.y = max3f(best.y, b0, b1);
                     }
                 }
             }
         }
+        xfer[role * 32 + lane] = best;
+        if constexpr (ROT) xrot[role * 32 + lane] = brot;
+        __syncthreads();
     }
-    // merge the role-0 lists with the particle's running top-8 (lowest id among equal
-    // correlations); the slab space holds the candidates now
-    __syncthreads();
-    float *ccs = reinterpret_cast<float *>(smem4);                 // [8 ROWS + 8]
-    int *ids = reinterpret_cast<int *>(ccs + 8 * ROWS + 8);
-    if (role == 0) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) { ccs[8 * lr + k] = kc[k]; ids[8 * lr + k] = ki[k]; }
-    }
+    if (role != NR - 1) return;
+    merge(pr0 + (pr1 - pr0) / 32 * 32);
+    // the lanes' lists and the particle's running top 8, whose slots follow them (lowest id among
+    // equal correlations)
+    __syncwarp();
     float2 *cp = cand + (size_t)(w_col0 + cl) * 8;
-    if (t < 8) {
-        const float2 c = cp[t];
-        ccs[8 * ROWS + t] = c.x;
-        ids[8 * ROWS + t] = __float_as_int(c.y);
+    float pc = -INFINITY;
+    int pid = 0x7fffffff;
+    if (lane < 8) {
+        const float2 c = cp[lane];
+        pc = c.x;
+        pid = __float_as_int(c.y);
     }
-    __syncthreads();
-    if (t < 32) {
-        const int n = 8 * ROWS + 8;
-        float keep_c = -INFINITY;
-        int keep_i = -1;
-        for (int it = 0; it < 8; ++it) {
-            float bc = -INFINITY;
-            int bi = 0x7fffffff, bpos = -1;
-            for (int e = t; e < n; e += 32) {
-                const float c = ccs[e];
-                const int id = ids[e];
-                if (c != -INFINITY && ranks_above(c, id, bc, bi)) { bc = c; bi = id; bpos = e; }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const float oc = __shfl_xor_sync(0xffffffffu, bc, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                const int op = __shfl_xor_sync(0xffffffffu, bpos, o);
-                if (ranks_above(oc, oi, bc, bi)) { bc = oc; bi = oi; bpos = op; }
-            }
-            if (t == it) { keep_c = bc; keep_i = bc == -INFINITY ? -1 : bi; }
-            if (bpos >= 0 && t == (bpos & 31)) ccs[bpos] = -INFINITY;
-            __syncwarp();
+    float keep_c = -INFINITY;
+    int keep_i = -1, head = 0;   // each lane's list is sorted: its head is its best
+    for (int it = 0; it < 8; ++it) {
+        float bc = head < 8 ? kc[head * 32 + lane] : -INFINITY;
+        int bi = head < 8 ? ki[head * 32 + lane] : 0x7fffffff;
+        if (bc == -INFINITY) bi = 0x7fffffff;
+        const bool old = pc != -INFINITY && ranks_above(pc, pid, bc, bi);
+        if (old) { bc = pc; bi = pid; }
+        float mc = bc;
+        int mi = bi;
+        for (int o = 16; o > 0; o >>= 1) {
+            const float oc = __shfl_xor_sync(0xffffffffu, mc, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, mi, o);
+            if (ranks_above(oc, oi, mc, mi)) { mc = oc; mi = oi; }
         }
-        if (t < 8) cp[t] = make_float2(keep_c, __int_as_float(keep_i));
+        if (lane == it) { keep_c = mc; keep_i = mc == -INFINITY ? -1 : mi; }
+        if (mc != -INFINITY && bc == mc && bi == mi) {   // ids are distinct: one lane's
+            if (old) pc = -INFINITY; else ++head;
+        }
     }
+    if (lane < 8) cp[lane] = make_float2(keep_c, __int_as_float(keep_i));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -926,46 +830,51 @@ static void fill_tw(TwTables &tw, int P)
 
 bool stage2_fast_supported(int P) { return P == 64 || P == 180 || P == 300; }
 
-// the inner factor P2 of the split P = P1 x P2 used for each supported length
-int stage2_fast_p2(int P) { return P == 64 ? 8 : P == 180 ? 15 : P == 300 ? 20 : 0; }
-
-// floats of normalising factors per (reference, particle) the search's pass B reads
+// floats of normalising factors per (reference, particle) the search's pass B reads, and the group
+// layout k_norm_fft writes them in (S2Split)
 int stage2_fast_dlen(int P)
 {
     switch (P) {
-    case 64: return s2_dlen<8, 8>();
-    case 180: return s2_dlen<12, 15>();
-    case 300: return s2_dlen<15, 20>();
+    case 64: return s2_dlen<64>();
+    case 180: return s2_dlen<180>();
+    case 300: return s2_dlen<300>();
     default: return P;
     }
 }
 
-template <int P1, int P2>
-static cudaError_t launch_s2(pftcc_handle *h, const S2Fast &sp, int blocks, const S2Wave *waves_dev, float2 *cand,
-                             float *ccall, const int *perm, bool eu)
+template <int P, bool ROT, bool WRITE, bool EU>
+static cudaError_t launch_s2_k(pftcc_handle *h, const S2Fast &sp, int blocks, const S2Wave *waves_dev, float2 *cand,
+                               float *ccall, const int *perm)
 {
+    using S = S2Split<P>;
     TwTables tw;
-    fill_tw(tw, P1 * P2);
-    // row slabs of P complex (the two-lane layout): 128 rows in flight up to P = 200, 64
-    // beyond; NT threads per row
-    constexpr int ROWS = P1 * P2 <= 200 ? 128 : 64;
-    constexpr int NT = S2_THREADS_PER_ROW;
-    const size_t smem = (size_t)((P2 + 1) / 2) * P1 * 2 * ROWS * sizeof(float2) +
-                        (size_t)P1 * P2 * (sizeof(float4) + sizeof(float2)) +
-                        (size_t)(NT - 1) * ROWS * (sizeof(float) + sizeof(int));
-    auto kern = ccall ? (eu ? k_stage2_fast<P1, P2, ROWS, NT, true, true> : k_stage2_fast<P1, P2, ROWS, NT, true, false>)
-                      : (eu ? k_stage2_fast<P1, P2, ROWS, NT, false, true> : k_stage2_fast<P1, P2, ROWS, NT, false, false>);
-    cudaError_t e = smem_limit((const void *)kern, smem);
+    fill_tw(tw, P);
+    const size_t smem = (size_t)P * 32 * sizeof(float4) + (size_t)S::ROLES * 32 * (sizeof(float2) + (ROT ? sizeof(int2) : 0)) +
+                        8 * 32 * (sizeof(float) + sizeof(int));
+    const cudaError_t e = smem_limit((const void *)k_stage2_fast<P, ROT, WRITE, EU>, smem);
     if (e != cudaSuccess) return e;
     PFTCC_LAUNCH(h);
     KTimer kt(h, PFTCC_K_STAGE2);
-    kern<<<blocks, NT * ROWS, smem, h->stream>>>(sp, tw, waves_dev, cand, ccall, perm);
+    k_stage2_fast<P, ROT, WRITE, EU><<<blocks, 32 * S::ROLES, smem, h->stream>>>(sp, tw, waves_dev, cand, ccall, perm);
     return cudaGetLastError();
 }
 
-// every wave of the list in one launch, one block per column (blk0 filled in)
+template <int P>
+static cudaError_t launch_s2(pftcc_handle *h, const S2Fast &sp, int blocks, const S2Wave *waves_dev, float2 *cand,
+                             float *ccall, const int *perm, bool eu, bool rot)
+{
+    if (ccall) return eu ? launch_s2_k<P, true, true, true>(h, sp, blocks, waves_dev, cand, ccall, perm)
+                         : launch_s2_k<P, true, true, false>(h, sp, blocks, waves_dev, cand, ccall, perm);
+    if (rot) return eu ? launch_s2_k<P, true, false, true>(h, sp, blocks, waves_dev, cand, ccall, perm)
+                       : launch_s2_k<P, true, false, false>(h, sp, blocks, waves_dev, cand, ccall, perm);
+    return eu ? launch_s2_k<P, false, false, true>(h, sp, blocks, waves_dev, cand, ccall, perm)
+              : launch_s2_k<P, false, false, false>(h, sp, blocks, waves_dev, cand, ccall, perm);
+}
+
+// every wave of the list in one launch, one block per column (blk0 filled in); rot: the candidates
+// carry their rotation (nothing re-scores them)
 cudaError_t launch_stage2_waves(pftcc_handle *h, int P, std::vector<S2Wave> &waves, int nshifts, int nrs_total,
-                                float2 *cand, float *ccall, const int *perm, int eu)
+                                float2 *cand, float *ccall, const int *perm, int eu, int rot)
 {
     UmmaState &us = h->ws.umma;
     const int nw = (int)waves.size();
@@ -973,7 +882,7 @@ cudaError_t launch_stage2_waves(pftcc_handle *h, int P, std::vector<S2Wave> &wav
     long long blocks = 0;
     for (S2Wave &w : waves) {
         if ((unsigned long long)P * w.xcols * w.xrows >= (1ull << 32) || w.cols <= 0 || w.rows <= 0 ||
-            w.zc0 + w.cols > w.xcols || w.rofs + w.rows > w.xrows)
+            w.zc0 + w.cols > w.xcols || w.rofs + w.rows > w.xrows || (w.xrows & 1))
             return cudaErrorInvalidValue;
         w.blk0 = (int)blocks;
         blocks += w.cols;
@@ -992,20 +901,20 @@ cudaError_t launch_stage2_waves(pftcc_handle *h, int P, std::vector<S2Wave> &wav
         return cudaErrorInvalidValue;
     S2Fast sp{nshifts, 2 * P, nrs_total, nw, 1.0f / (2.0f * (float)(2 * P))};
     switch (P) {
-    case 64: return launch_s2<8, 8>(h, sp, (int)blocks, us.d_s2waves, cand, ccall, perm, eu != 0);
-    case 180: return launch_s2<12, 15>(h, sp, (int)blocks, us.d_s2waves, cand, ccall, perm, eu != 0);
-    case 300: return launch_s2<15, 20>(h, sp, (int)blocks, us.d_s2waves, cand, ccall, perm, eu != 0);
+    case 64: return launch_s2<64>(h, sp, (int)blocks, us.d_s2waves, cand, ccall, perm, eu != 0, rot != 0);
+    case 180: return launch_s2<180>(h, sp, (int)blocks, us.d_s2waves, cand, ccall, perm, eu != 0, rot != 0);
+    case 300: return launch_s2<300>(h, sp, (int)blocks, us.d_s2waves, cand, ccall, perm, eu != 0, rot != 0);
     default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_stage2_fast(pftcc_handle *h, int P, int rows, int xrows, int xcols, int row0, int nshifts, int r0,
                                int dcols, int col0, int cols, int nrs_total, const float2 *X, const float *Dinv,
-                               float2 *cand, float *ccall, const int *perm, int eu)
+                               float2 *cand, float *ccall, const int *perm, int eu, int rot)
 {
     std::vector<S2Wave> w(1);
     w[0] = S2Wave{X, Dinv, row0, rows, 0, xrows, xcols, col0, cols, 0, r0, dcols, 0, 0};
-    return launch_stage2_waves(h, P, w, nshifts, nrs_total, cand, ccall, perm, eu);
+    return launch_stage2_waves(h, P, w, nshifts, nrs_total, cand, ccall, perm, eu, rot);
 }
 
 template <int P1, int P2, bool EU>

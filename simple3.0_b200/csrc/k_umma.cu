@@ -28,7 +28,7 @@
 //   warps 2-9 epilogue, two per TMEM lane quadrant (warp w: quadrant w mod 4, half
 //            (w - 2) / 4 of the tile): tcgen05.ld of its 16 (ref, shift) rows of both
 //            planes' accumulators, Z(m) and Z(P - m) into two 128B-swizzled staging tiles,
-//            written out with one TMA bulk store each to Z[plane][col][rs]
+//            written out with one TMA bulk store each to Z[plane][col][row pair] (re, re, im, im)
 // The factor 4 of X is carried by the packed particle operand (exact in BF16).
 // Every mbarrier wait is bounded; on timeout the kernel records an error code,
 // drains its own outstanding copies (bounded), frees its TMEM and returns.  The pipeline
@@ -404,10 +404,10 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_umma_stage1(const __grid_const
                             xa0.y = xa1.y = xb0.y = xb1.y = 0.f;
                         }
                         const float2 za0 = make_z(xa0, xb0, wA), za1 = make_z(xa1, xb1, wA);
-                        rowA[e ^ (lane & 7)] = make_float4(za0.x, za0.y, za1.x, za1.y);
+                        rowA[e ^ (lane & 7)] = make_float4(za0.x, za1.x, za0.y, za1.y);   // a row pair: re, re, im, im
                         if (two) {
                             const float2 zb0 = make_z(xb0, xa0, wB), zb1 = make_z(xb1, xa1, wB);
-                            rowB[e ^ (lane & 7)] = make_float4(zb0.x, zb0.y, zb1.x, zb1.y);
+                            rowB[e ^ (lane & 7)] = make_float4(zb0.x, zb1.x, zb0.y, zb1.y);
                         }
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -528,7 +528,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 get_encode()
     return fn;
 }
 
-// X[M][xcols][xrows] float2 as a 2-D FP32 tensor: x = 2 * rs + (re, im), y = m * xcols + col;
+// X[M][xcols][xrows] float2 as a 2-D FP32 tensor: x = four floats (re, re, im, im) a row pair, y = m * xcols + col;
 // boxes of 32 floats (128 B) x 32 rows, 128-byte swizzle (the staging layout of the epilogue)
 static int make_xmap(pftcc_handle *h, CUtensorMap *map, void *X, int xrows, int xcols, int nplanes)
 {
