@@ -9,6 +9,7 @@
 // rotations that k_exact_fft.cu has no transform for.
 #include "pftcc_internal.cuh"
 
+#include <algorithm>
 #include <cstddef>
 #include <cmath>
 
@@ -463,32 +464,10 @@ cudaError_t launch_exact(pftcc_handle *h, const Group *groups, int ngroups, cons
 // precision: gencorr_cc_for_rot_8 (:1690-1733) and gencorr_cc_grad_for_rot_8
 // (:1863-1925), both branches (match_filt: unweighted sums normalised with
 // sqsums over kstop; otherwise shell weights k in numerator and both norms).
-// The derivative with respect to the defocus multiplies the reference by
-// d|CTF|/d(df) instead of |CTF| and applies the quotient rule to the norm.
-//
-// One block per request.  ctf_mode 0: stored ctfmats (the drop-in calls);
-// ctf_mode 1: |CTF| and its derivative recomputed at defocus + ddf.
+// The drop-in calls and the shift search: the stored |CTF| matrices, one block per request.
 struct RotReq { int iref, slot, irot, ctf_mode; double sx, sy, ddf; };
 static_assert(sizeof(RotReq) == sizeof(RotReqH) && offsetof(RotReq, sx) == offsetof(RotReqH, sx),
               "RotReqH mirrors RotReq");
-
-__device__ __forceinline__ double ctf_abs_d(const pftcc_ctfparams &c, double s2, double ang, double ddf, double *dctf)
-{
-    const double kv = 1000.0 * (double)c.kv;
-    const double wl = (12.26 / sqrt(kv + (0.9784 * kv * kv) / 1.0e6)) / (double)c.smpd;
-    const double cs = ((double)c.cs * 1.0e7) / (double)c.smpd;
-    const double ampc = atan((double)c.fraca / sqrt(1.0 - (double)c.fraca * c.fraca));
-    const double sc = 1.0e4 / (double)c.smpd;
-    const double dfx = ((double)c.dfx + ddf) * sc, dfy = ((double)c.dfy + ddf) * sc;
-    const double angast = (double)c.angast / 180.0 * 3.141592653589793;
-    const double df = 0.5 * (dfx + dfy + cos(2.0 * (ang - angast)) * (dfx - dfy));
-    double chi = 3.141592653589793 * wl * s2 * (df - 0.5 * wl * wl * s2 * cs) + ampc;
-    if (c.l_phaseplate) chi += (double)c.phshift;
-    double s, co;
-    sincos(chi, &s, &co);
-    *dctf = (s >= 0.0 ? 1.0 : -1.0) * co * 3.141592653589793 * wl * s2 * sc;
-    return fabs(s);
-}
 
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double *red)
@@ -508,9 +487,9 @@ constexpr int FR_THREADS = 256;
 __global__ void __launch_bounds__(FR_THREADS) k_for_rot(
     Geom g, const RotReq *__restrict__ reqs, const float2 *__restrict__ refs_even,
     const float2 *__restrict__ refs_odd, const float2 *__restrict__ ptcls, const float *__restrict__ ctfmats,
-    const pftcc_ctfparams *__restrict__ ctfp, const uint8_t *__restrict__ iseven, const float *__restrict__ polar,
-    const double *__restrict__ argtransf, const double *__restrict__ argtransf1, int with_ctf, int match_filt,
-    const float *__restrict__ snorm, int nrefs, double *__restrict__ out /* [nreq][5]: f, d/dsx, d/dsy, d/ddf, unused */)
+    const uint8_t *__restrict__ iseven, const double *__restrict__ argtransf, const double *__restrict__ argtransf1,
+    int with_ctf, int match_filt, const float *__restrict__ snorm, int nrefs,
+    double *__restrict__ out /* [nreq][5]: f, d/dsx, d/dsy, 0, unused */)
 {
     __shared__ double red[FR_THREADS / 32];
     const RotReq rq = reqs[blockIdx.x];
@@ -520,7 +499,7 @@ __global__ void __launch_bounds__(FR_THREADS) k_for_rot(
     // matched-filter mode: shellnorm_and_filter_ref_8's factors
     const float *sn = snorm ? snorm + ((size_t)(iseven[rq.slot] ? 0 : 1) * nrefs + rq.iref) * g.Ks : nullptr;
     const int s = rq.irot - 1;
-    double corr = 0, sqr = 0, sqp = 0, gx = 0, gy = 0, gd = 0, dsq = 0;
+    double corr = 0, sqr = 0, sqp = 0, gx = 0, gy = 0;
     // thread per n; the shift phase of every shell follows the de Moivre recurrence
     for (int n = threadIdx.x; n < P; n += blockDim.x) {
         const double a = argtransf[n] * rq.sx + argtransf[P + n] * rq.sy;
@@ -534,16 +513,7 @@ __global__ void __launch_bounds__(FR_THREADS) k_for_rot(
         const double qs = j < P ? 1.0 : -1.0;
         for (int ik = 0; ik < g.Ks; ++ik) {
             const double wgt = match_filt ? 1.0 : (double)(g.kfrom + ik);
-            double c = 1.0, dc = 0.0;
-            if (with_ctf) {
-                if (rq.ctf_mode == 0) {
-                    c = (double)ctfmats[((long long)rq.slot * g.K + ik) * P + n];
-                } else {
-                    const double x = polar[ik * 2 * N + n], y = polar[ik * 2 * N + N + n];
-                    const double hinv = x / g.box, kinv = y / g.box;
-                    c = ctf_abs_d(ctfp[rq.slot], hinv * hinv + kinv * kinv, atan2(y, x), rq.ddf, &dc);
-                }
-            }
+            const double c = with_ctf ? (double)ctfmats[((long long)rq.slot * g.K + ik) * P + n] : 1.0;
             const float2 rv = r[(long long)ik * P + n];
             const double f = sn ? (double)sn[ik] : 1.0;
             const double rr = (double)rv.x * f * c, ri = (double)rv.y * f * c;
@@ -557,12 +527,6 @@ __global__ void __launch_bounds__(FR_THREADS) k_for_rot(
             const double ax = argtransf[ik * N + n], ay = argtransf[ik * N + P + n];
             gx += wgt * ax * (-ai * qr + ar * qi);
             gy += wgt * ay * (-ai * qr + ar * qi);
-            if (with_ctf && rq.ctf_mode == 1) {
-                const double dr = (double)rv.x * f * dc, di = (double)rv.y * f * dc;
-                const double br = dr * st_r - di * st_i, bi = dr * st_i + di * st_r;
-                gd += wgt * (br * qr + bi * qi);
-                dsq += wgt * 2.0 * (ar * br + ai * bi);
-            }
             const double nr = st_r * v_r - st_i * v_i, ni = st_r * v_i + st_i * v_r;
             st_r = nr; st_i = ni;
         }
@@ -572,8 +536,6 @@ __global__ void __launch_bounds__(FR_THREADS) k_for_rot(
     sqp = block_sum<FR_THREADS>(sqp, red);
     gx = block_sum<FR_THREADS>(gx, red);
     gy = block_sum<FR_THREADS>(gy, red);
-    gd = block_sum<FR_THREADS>(gd, red);
-    dsq = block_sum<FR_THREADS>(dsq, red);
     if (threadIdx.x == 0) {
         const double den = sqrt(sqr * sqp);
         const double f = corr / den;
@@ -581,7 +543,7 @@ __global__ void __launch_bounds__(FR_THREADS) k_for_rot(
         o[0] = f;
         o[1] = gx / den;
         o[2] = gy / den;
-        o[3] = (with_ctf && rq.ctf_mode == 1) ? (gd / den - 0.5 * f * dsq / sqr) : 0.0;
+        o[3] = 0.0;
         o[4] = 0.0;
     }
 }
@@ -596,8 +558,8 @@ cudaError_t launch_for_rot(pftcc_handle *h, int iref, int slot, double sx, doubl
     if (e != cudaSuccess) return e;
     PFTCC_LAUNCH(h);
     k_for_rot<<<1, FR_THREADS, 0, h->stream>>>(h->g, reinterpret_cast<const RotReq *>(h->d_work), h->refs_even,
-                                                h->refs_odd, h->ptcls, h->ctfmats, h->d_ctfp, h->d_iseven, h->polar,
-                                                h->argtransf, h->argtransf1, h->cfg.with_ctf && h->ctf_ready,
+                                                h->refs_odd, h->ptcls, h->ctfmats, h->d_iseven, h->argtransf,
+                                                h->argtransf1, h->cfg.with_ctf && h->ctf_ready,
                                                 match_filt, snorm_ptr(h), h->nrefs, out5);
     return cudaGetLastError();
 }
@@ -608,8 +570,8 @@ cudaError_t launch_rot_reqs(pftcc_handle *h, const void *reqs_dev, int n, double
 {
     PFTCC_LAUNCH(h);
     k_for_rot<<<n, FR_THREADS, 0, h->stream>>>(h->g, reinterpret_cast<const RotReq *>(reqs_dev), h->refs_even,
-                                                h->refs_odd, h->ptcls, h->ctfmats, h->d_ctfp, h->d_iseven, h->polar,
-                                                h->argtransf, h->argtransf1, h->cfg.with_ctf && h->ctf_ready,
+                                                h->refs_odd, h->ptcls, h->ctfmats, h->d_iseven, h->argtransf,
+                                                h->argtransf1, h->cfg.with_ctf && h->ctf_ready,
                                                 h->cfg.match_filt, snorm_ptr(h), h->nrefs, out5);
     return cudaGetLastError();
 }
@@ -708,27 +670,171 @@ cudaError_t launch_specscore(pftcc_handle *h, const FrcReq *reqs_dev, int nreq, 
     return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// The adjoint: gencorr_cc_grad_for_rot_8 with |CTF| recomputed at defocus + ddf and the derivative by the
+// defocus too, which multiplies the reference by d|CTF|/d(df) instead of |CTF| and applies the
+// quotient rule to the norm.  One block per request.
+// |CTF| of one request over the grid: with hx, hy the sample's frequencies (cycles per pixel of the box),
+//   chi = pi wl s2 (df - wl^2 s2 cs / 2) + phi0,  df = (dfx + dfy + cos(2 (ang - angast)) (dfx - dfy)) / 2,
+// and s2 cos(2 (ang - angast)) = (hx^2 - hy^2) cos(2 angast) + 2 hx hy sin(2 angast), so that
+//   chi = s2 (a - c s2) + bc (hx^2 - hy^2) + bs 2 hx hy + phi0,  d chi / d(defocus) = d s2:
+// the angle's arctangent and cosine and every constant of the optics leave the samples' loop
+struct RotCtf { double a, bc, bs, c, phi0, d; };
+
+__device__ __forceinline__ RotCtf rot_ctf(const pftcc_ctfparams &p, double ddf)
+{
+    const double pi = 3.141592653589793;
+    const double kv = 1000.0 * (double)p.kv;
+    const double wl = (12.26 / sqrt(kv + (0.9784 * kv * kv) / 1.0e6)) / (double)p.smpd;
+    const double cs = ((double)p.cs * 1.0e7) / (double)p.smpd;
+    const double sc = 1.0e4 / (double)p.smpd;
+    const double dfx = ((double)p.dfx + ddf) * sc, dfy = ((double)p.dfy + ddf) * sc;
+    const double angast = (double)p.angast / 180.0 * pi;
+    double s2a, c2a;
+    sincos(2.0 * angast, &s2a, &c2a);
+    RotCtf r;
+    r.a = pi * wl * 0.5 * (dfx + dfy);
+    r.bc = pi * wl * 0.5 * (dfx - dfy) * c2a;
+    r.bs = pi * wl * 0.5 * (dfx - dfy) * s2a;
+    r.c = pi * wl * 0.5 * wl * wl * cs;
+    r.phi0 = atan((double)p.fraca / sqrt(1.0 - (double)p.fraca * p.fraca)) + (p.l_phaseplate ? (double)p.phshift : 0.0);
+    r.d = pi * wl * sc;
+    return r;
+}
+
+constexpr int FR_MAX = 384;           // k_adjoint's largest block
+
+// The block: segments of ceil32(P) threads, thread per n, each segment a share of the shells (two at
+// P = 180, six at 64): every warp is full but the last of a segment, and a single request has the most
+// threads its samples allow.  What bounds it: the FP64 pipe -- about 30 operations a sample and the
+// sine and cosine of the CTF (CTF false: none).
+// 22,000 requests at P = 180, Ks = 39 (recomputed CTF): before, with the arctangent, cosine and optics
+// constants in the loop, seven block sums and 180 of 256 threads, 7.8 ms; now 2.2.
+template <bool CTF>
+__global__ void __launch_bounds__(FR_MAX) k_adjoint(
+    Geom g, int tp, const RotReq *__restrict__ reqs, const RotCtf *__restrict__ rctf, const float2 *__restrict__ refs_even,
+    const float2 *__restrict__ refs_odd, const float2 *__restrict__ ptcls, const uint8_t *__restrict__ iseven, const float *__restrict__ polar,
+    const double *__restrict__ argtransf, const double *__restrict__ argtransf1, int match_filt,
+    const float *__restrict__ snorm, int nrefs, double *__restrict__ out /* [nreq][5]: f, d/dsx, d/dsy, d/ddf, unused */)
+{
+    __shared__ double red[7][FR_MAX / 32];
+    const RotReq rq = reqs[blockIdx.x];
+    const int N = g.N, P = g.P, nseg = blockDim.x / tp;
+    const float2 *q = ptcls + (long long)rq.slot * g.K * P;
+    const float2 *r = (iseven[rq.slot] ? refs_even : refs_odd) + (long long)rq.iref * g.K * P;
+    // matched-filter mode: shellnorm_and_filter_ref_8's factors
+    const float *sn = snorm ? snorm + ((size_t)(iseven[rq.slot] ? 0 : 1) * nrefs + rq.iref) * g.Ks : nullptr;
+    const int seg = threadIdx.x / tp, n0 = threadIdx.x - seg * tp;
+    const int ka = seg * g.Ks / nseg, kz = (seg + 1) * g.Ks / nseg;
+    const double inv_box = 1.0 / (double)g.box, A = 3.141592653589793 / (double)(g.box / 2);   // argtransf = polar A
+    RotCtf cp{};
+    if (CTF) cp = rctf[blockIdx.x];
+    double v[7] = {0, 0, 0, 0, 0, 0, 0};   // corr, |A|^2, |ptcl|^2, d/dsx, d/dsy, d corr/ddf, d |A|^2/ddf over 2
+    for (int n = n0; n < P; n += tp) {
+        // the shift phase of the segment's first shell, then the de Moivre recurrence
+        double st_r, st_i, v_r, v_i;
+        const double a1 = argtransf1[n] * rq.sx + argtransf1[P + n] * rq.sy;
+        sincos(argtransf[n] * rq.sx + argtransf[P + n] * rq.sy + ka * a1, &st_i, &st_r);
+        sincos(a1, &v_i, &v_r);
+        int j = rq.irot - 1 + n;
+        if (j >= N) j -= N;
+        const int jp = j < P ? j : j - P;
+        const float qs = j < P ? 1.f : -1.f;
+#pragma unroll 2
+        for (int ik = ka; ik < kz; ++ik) {
+            const double wgt = match_filt ? 1.0 : (double)(g.kfrom + ik);
+            const double x = polar[ik * 2 * N + n], y = polar[ik * 2 * N + N + n];
+            const float2 rv = r[(long long)ik * P + n], qv = q[(long long)ik * P + jp];
+            double c = 1.0, dc = 0.0;
+            if (CTF) {
+                const double hx = x * inv_box, hy = y * inv_box, u = hx * hx, w = hy * hy, s2 = u + w;
+                const double chi = s2 * (cp.a - cp.c * s2) + cp.bc * (u - w) + cp.bs * (2.0 * hx * hy) + cp.phi0;
+                double s, co;
+                sincos(chi, &s, &co);
+                c = fabs(s);
+                dc = (s >= 0.0 ? co : -co) * cp.d * s2;
+            }
+            double rr = rv.x, ri = rv.y;
+            if (sn) { rr *= (double)sn[ik]; ri *= (double)sn[ik]; }
+            const double pr = rr * st_r - ri * st_i, pi = rr * st_i + ri * st_r;   // the reference times the phase
+            const double q0r = qv.x, q0i = (double)(qs * qv.y), qr = wgt * q0r, qi = wgt * q0i;   // ptcl~(j), weighted
+            const double e1 = pr * qr + pi * qi, e2 = c * (pr * qi - pi * qr);
+            const double m = wgt * (pr * pr + pi * pi), cm = c * m;
+            v[0] += c * e1;
+            v[1] += c * cm;
+            v[2] += q0r * qr + q0i * qi;
+            v[3] += x * e2;       // argtransf_x = x A: Re sum i argtransf A conj(ptcl~)
+            v[4] += y * e2;
+            if (CTF) {
+                v[5] += dc * e1;
+                v[6] += dc * cm;
+            }
+            const double nr = st_r * v_r - st_i * v_i, ni = st_r * v_i + st_i * v_r;
+            st_r = nr; st_i = ni;
+        }
+    }
+    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        if (!CTF && i >= 5) continue;
+        for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+        if ((threadIdx.x & 31) == 0) red[i][warp] = v[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 7; ++i) {
+            v[i] = 0.0;
+            if (CTF || i < 5)
+                for (int w = 0; w < nw; ++w) v[i] += red[i][w];
+        }
+        const double den = sqrt(v[1] * v[2]);
+        const double f = v[0] / den;
+        double *o = out + 5 * blockIdx.x;
+        o[0] = f;
+        o[1] = A * v[3] / den;
+        o[2] = A * v[4] / den;
+        o[3] = CTF ? v[5] / den - f * v[6] / v[1] : 0.0;
+        o[4] = 0.0;
+    }
+}
+
+// n requests on the device and their CTF constants
+static cudaError_t launch_adjoint(pftcc_handle *h, const RotReq *reqs, const RotCtf *rctf, int n, int match_filt,
+                                    double *out5)
+{
+    const int tp = std::min(FR_MAX, (h->g.P + 31) / 32 * 32), nseg = std::max(1, std::min(FR_MAX / tp, h->g.Ks));
+    auto k = h->cfg.with_ctf && h->ctf_ready ? k_adjoint<true> : k_adjoint<false>;
+    PFTCC_LAUNCH(h);
+    k<<<n, nseg * tp, 0, h->stream>>>(h->g, tp, reqs, rctf, h->refs_even, h->refs_odd, h->ptcls, h->d_iseven,
+                                      h->polar, h->argtransf, h->argtransf1, match_filt, snorm_ptr(h), h->nrefs, out5);
+    return cudaGetLastError();
+}
+
+// the adjoint's requests and their CTF constants
 __global__ void k_grad_reqs(const pftcc_grad_req *__restrict__ in, const int *__restrict__ slots, int n,
-                            RotReq *__restrict__ out)
+                            const pftcc_ctfparams *__restrict__ ctfp, int with_ctf, RotReq *__restrict__ out,
+                            RotCtf *__restrict__ rctf)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const pftcc_grad_req r = in[i];
     out[i] = RotReq{r.iref - 1, slots[i], r.irot, 1, r.sx, r.sy, r.ddf};
+    if (with_ctf) rctf[i] = rot_ctf(ctfp[slots[i]], r.ddf);
 }
+
+size_t grad_work_bytes(int nreq) { return (size_t)nreq * (sizeof(RotReq) + sizeof(RotCtf)); }
 
 cudaError_t launch_grad_batch(pftcc_handle *h, const pftcc_grad_req *req_dev, const int *slots_dev, int nreq,
                               double *out5)
 {
-    RotReq *rq = reinterpret_cast<RotReq *>(h->d_work);
+    RotCtf *rc = reinterpret_cast<RotCtf *>(h->d_work);
+    RotReq *rq = reinterpret_cast<RotReq *>(rc + nreq);
     PFTCC_LAUNCH(h);
-    k_grad_reqs<<<(nreq + 255) / 256, 256, 0, h->stream>>>(req_dev, slots_dev, nreq, rq);
-    PFTCC_LAUNCH(h);
-    k_for_rot<<<nreq, FR_THREADS, 0, h->stream>>>(h->g, rq, h->refs_even, h->refs_odd, h->ptcls, h->ctfmats,
-                                                   h->d_ctfp, h->d_iseven, h->polar, h->argtransf, h->argtransf1,
-                                                   h->cfg.with_ctf && h->ctf_ready, h->cfg.match_filt, snorm_ptr(h),
-                                                   h->nrefs, out5);
-    return cudaGetLastError();
+    k_grad_reqs<<<(nreq + 63) / 64, 64, 0, h->stream>>>(req_dev, slots_dev, nreq, h->d_ctfp, h->cfg.with_ctf && h->ctf_ready,
+                                                        rq, rc);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return launch_adjoint(h, rq, rc, nreq, h->cfg.match_filt, out5);
 }
 
 }  // namespace pftcc

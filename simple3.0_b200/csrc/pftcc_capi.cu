@@ -1996,7 +1996,7 @@ int pftcc::grad_batch_host(pftcc_handle *h, int nreq, const pftcc_grad_req *req,
     }
     // device layout: [req][slots][RotReq work area][out]
     const size_t rq_bytes = (size_t)nreq * sizeof(pftcc_grad_req);
-    ST(ensure(h, (void **)&h->d_work, &h->work_cap, std::max<size_t>((size_t)nreq * 48, 4096), "grad work"));
+    ST(ensure(h, (void **)&h->d_work, &h->work_cap, std::max<size_t>(grad_work_bytes(nreq), 4096), "grad work"));
     ST(ensure(h, (void **)&h->d_dout, &h->dout_cap, (size_t)nreq * 5 * sizeof(double) + rq_bytes + (size_t)nreq * 4 + 64,
               "grad out"));
     char *base = (char *)h->d_dout;
