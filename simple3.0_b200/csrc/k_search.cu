@@ -219,28 +219,40 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_ptcl(
     }
 }
 
-// The same spectra by FP64 transforms of length N = N1 * N2 (spec_fft.cuh), shells in
-// batches of sfft::KB: (reference, shift) rows UA[m][rs][k], one block per row.  The shifted
+// The same spectra by FP64 transforms of length P = P1 * P2, two shells in each (spec_fft.cuh),
+// shells in batches of sfft::KB: (reference, shift) rows UA[m][rs][k], one block per row.  The shifted
 // polar samples a(n, k) are formed exactly as in k_spec_ref (FP32 products with the
 // single-precision shift phases of the de Moivre recurrence), a batch of shells at a time
 // ([shell][n] in shared memory), the recurrence state kept per angular sample n.
-template <int N1, int N2>
-__global__ void __launch_bounds__(SPEC_THREADS) k_spec_ref_fft(
-    Geom g, int nshifts, const float2 *__restrict__ refs, const float *__restrict__ shifts,
-    const double *__restrict__ argtransf, const double *__restrict__ argtransf1, int rs0, int nrs, int rows_pad,
-    float2 *__restrict__ UA, int kb_per_block)
+// wn: the table w_N^{-e}, e < N.  What bounds these kernels: the latency of the FP64 chains and the block's
+// barriers (60 to 96 KB of rows and samples a block, two blocks an SM).  With one transform of length N a
+// shell before: the references of 100 x 81 rows, P = 180, 2.16 ms, now 1.25; the particles of 5130 at
+// P = 300, 3.70 and 2.26, 1000 at P = 64, 0.063 and 0.053.
+template <int P> __device__ __forceinline__ void spec_tables(const double2 *__restrict__ wn, double2 *tn, double2 *tp)
 {
-    constexpr int N = N1 * N2, P = N / 2, NPT = (P + SPEC_THREADS - 1) / SPEC_THREADS;
+    for (int e = threadIdx.x; e < P; e += blockDim.x) {
+        tn[e] = wn[e];       // w_N^{-e}
+        tp[e] = wn[2 * e];   // w_P^{-e}
+    }
+}
+
+template <int P1, int P2>
+__global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ref_fft(
+    Geom g, int nshifts, const float2 *__restrict__ refs, const float *__restrict__ shifts,
+    const double *__restrict__ argtransf, const double *__restrict__ argtransf1, const double2 *__restrict__ wn, int nrs,
+    int rows_pad, float2 *__restrict__ UA, int kb_per_block)
+{
+    using R = sfft::Rows<P1, P2>;
+    constexpr int P = P1 * P2, NPT = (P + SPEC_THREADS - 1) / SPEC_THREADS, NP = sfft::KB / 2;
     extern __shared__ float4 smem4[];
     const int Ks = g.Ks, M = P + 1;
     // this block's shells [ka, kz): blockIdx.y selects kb_per_block batches of sfft::KB
     const int ka = blockIdx.y * kb_per_block * sfft::KB, kz = min(Ks, ka + kb_per_block * sfft::KB);
-    double2 *tw = reinterpret_cast<double2 *>(smem4);                              // [N] w_N^{-e}
-    double2 *buf = tw + N;                                                          // the transform buffer
-    float2 *a = reinterpret_cast<float2 *>(buf + sfft::buf_elems<N1, N2>());       // [KB][P]
+    double2 *tn = reinterpret_cast<double2 *>(smem4), *tp = tn + P;               // [P] w_N^{-e}, w_P^{-e}
+    double2 *buf = tp + P;                                                         // [2 NP] transforms' rows
+    float2 *a = reinterpret_cast<float2 *>(buf + 2 * NP * R::ROW);                 // [KB][P]
     const int row = blockIdx.x;
-    const int rs = rs0 + row;
-    if (rs >= nrs) {   // zero padding rows
+    if (row >= nrs) {   // zero padding rows
         const int nk = kz - ka;
         for (int e = threadIdx.x; e < M * nk; e += blockDim.x) {
             const int m = e / nk, k = ka + e - m * nk;
@@ -248,13 +260,9 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_ref_fft(
         }
         return;
     }
-    const int r = rs / nshifts, s = rs - r * nshifts;
-    for (int e = threadIdx.x; e < N; e += blockDim.x) {
-        double sn, cs;
-        sincospi(-2.0 * e / N, &sn, &cs);
-        tw[e] = make_double2(cs, sn);
-    }
-    const float2 *R = refs + (size_t)r * g.K * P;
+    const int r = row / nshifts, s = row - r * nshifts;
+    spec_tables<P>(wn, tn, tp);
+    const float2 *Rf = refs + (size_t)r * g.K * P;
     const double sx = shifts ? (double)shifts[2 * s] : 0.0, sy = shifts ? (double)shifts[2 * s + 1] : 0.0;
     // gen_shmat_8 per angular sample: analytic first shell, de Moivre recurrence over k
     double pr[NPT], pi[NPT], qr[NPT], qi[NPT];
@@ -279,44 +287,46 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_ref_fft(
             const int n = threadIdx.x + i * SPEC_THREADS;
             if (n >= P) continue;
             for (int kl = 0; kl < nk; ++kl) {
-                const float2 x = R[(size_t)(k0 + kl) * P + n];
+                const float2 x = Rf[(size_t)(k0 + kl) * P + n];
                 const float fr = (float)pr[i], fi = (float)pi[i];
                 a[kl * P + n] = make_float2(x.x * fr - x.y * fi, x.x * fi + x.y * fr);
                 const double nr = pr[i] * qr[i] - pi[i] * qi[i], ni = pr[i] * qi[i] + pi[i] * qr[i];
                 pr[i] = nr; pi[i] = ni;
             }
+            if (nk & 1) a[nk * P + n] = make_float2(0.f, 0.f);
         }
-        auto getf = [&](int kl, int n) {
-            const float2 v = a[kl * P + (n < P ? n : n - P)];
-            return make_double2((double)v.x, n < P ? (double)v.y : -(double)v.y);
-        };
-        auto put = [&](int kl, int m, double2 F) {
-            if (m <= P) {
-                const float2 u = (m & 1) ? make_float2((float)(0.5 * F.y), (float)(-0.5 * F.x))
-                                         : make_float2((float)(0.5 * F.x), (float)(0.5 * F.y));
-                UA[((size_t)m * rows_pad + row) * Ks + k0 + kl] = u;
-            }
-        };
-        sfft::batch_fft<N1, N2>(nk, getf, put, buf, tw);
+        R::run(2 * ((nk + 1) / 2), [&](int f, int n) {
+            const float2 u = a[(f & ~1) * P + n], v = a[(f | 1) * P + n];
+            return (f & 1) ? sfft::d_mul(make_double2((double)u.y, (double)v.y), tn[n]) : make_double2((double)u.x, (double)v.x);
+        }, buf, tp);
+        for (int e = threadIdx.x; e < M * NP; e += blockDim.x) {
+            const int q = e % NP, m = e / NP;
+            if (2 * q >= nk) continue;
+            double2 u, v;
+            R::pair(m, buf + 2 * q * R::ROW, buf + (2 * q + 1) * R::ROW, u, v);
+            float2 *dst = UA + ((size_t)m * rows_pad + row) * Ks + k0 + 2 * q;
+            dst[0] = make_float2((float)u.x, (float)u.y);
+            if (2 * q + 1 < nk) dst[1] = make_float2((float)v.x, (float)v.y);
+        }
     }
 }
 
 // particle-side spectra by the FP64 transforms: UB[m][col][k] of B = |CTF| * ptcl and the
-// CTF^2 spectra CV[col][j][k] = sum_{n<P} CTF^2(n, k) w_P^{-jn} (the even outputs F(2j) / 2
-// of the transform of the real sequence continued periodically over the full circle)
-template <int N1, int N2>
-__global__ void __launch_bounds__(SPEC_THREADS) k_spec_ptcl_fft(
+// CTF^2 spectra CV[col][j][k] = sum_{n<P} CTF^2(n, k) w_P^{-jn}, a third transform per shell pair
+template <int P1, int P2>
+__global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ptcl_fft(
     Geom g, const float2 *__restrict__ ptcls, const float *__restrict__ ctfmats, const int *__restrict__ perm,
-    int ncols, int cols_pad, float2 *__restrict__ UB, double2 *__restrict__ CV, float *__restrict__ sqp_out,
-    const float *__restrict__ sqsums, int kb_per_block)
+    const double2 *__restrict__ wn, int ncols, int cols_pad, float2 *__restrict__ UB, double2 *__restrict__ CV,
+    float *__restrict__ sqp_out, const float *__restrict__ sqsums, int kb_per_block)
 {
-    constexpr int N = N1 * N2, P = N / 2, J = P / 2 + 1;
+    using R = sfft::Rows<P1, P2>;
+    constexpr int P = P1 * P2, J = P / 2 + 1, NP = sfft::KB / 2;
     extern __shared__ float4 smem4[];
     const int Ks = g.Ks, M = P + 1;
     const int ka = blockIdx.y * kb_per_block * sfft::KB, kz = min(Ks, ka + kb_per_block * sfft::KB);
-    double2 *tw = reinterpret_cast<double2 *>(smem4);                              // [N]
-    double2 *buf = tw + N;
-    float2 *b = reinterpret_cast<float2 *>(buf + sfft::buf_elems<N1, N2>());       // [KB][P]
+    double2 *tn = reinterpret_cast<double2 *>(smem4), *tp = tn + P;               // [P] w_N^{-e}, w_P^{-e}
+    double2 *buf = tp + P;                                                         // [3 NP] transforms' rows
+    float2 *b = reinterpret_cast<float2 *>(buf + 3 * NP * R::ROW);                 // [KB][P]
     float *c2 = reinterpret_cast<float *>(b + sfft::KB * P);                        // [KB][P]
     const int col = blockIdx.x;
     if (col >= ncols) {
@@ -333,39 +343,44 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_ptcl_fft(
         return;
     }
     const int slot = perm[col];
-    for (int e = threadIdx.x; e < N; e += blockDim.x) {
-        double sn, cs;
-        sincospi(-2.0 * e / N, &sn, &cs);
-        tw[e] = make_double2(cs, sn);
-    }
+    spec_tables<P>(wn, tn, tp);
     const float2 *Q = ptcls + (size_t)slot * g.K * P;
     const float *C = ctfmats ? ctfmats + (size_t)slot * g.K * P : nullptr;
     if (threadIdx.x == 0 && blockIdx.y == 0) sqp_out[col] = sqsums[slot];
     for (int k0 = ka; k0 < kz; k0 += sfft::KB) {
         const int nk = min(sfft::KB, kz - k0);
-        for (int e = threadIdx.x; e < nk * P; e += blockDim.x) {   // e = kl P + n
-            const float c = C ? C[(size_t)k0 * P + e] : 1.f;
-            const float2 q = Q[(size_t)k0 * P + e];
+        for (int e = threadIdx.x; e < ((nk + 1) & ~1) * P; e += blockDim.x) {   // e = kl P + n; an odd shell's partner is 0
+            const bool in = e < nk * P;
+            const float c = in ? (C ? C[(size_t)k0 * P + e] : 1.f) : 0.f;
+            const float2 q = in ? Q[(size_t)k0 * P + e] : make_float2(0.f, 0.f);
             b[e] = make_float2(c * q.x, c * q.y);
             c2[e] = c * c;
         }
-        auto getf = [&](int kl, int n) {
-            const float2 v = b[kl * P + (n < P ? n : n - P)];
-            return make_double2((double)v.x, n < P ? (double)v.y : -(double)v.y);
-        };
-        auto put = [&](int kl, int m, double2 F) {
-            if (m <= P) {
-                const float2 u = (m & 1) ? make_float2((float)(0.5 * F.y), (float)(-0.5 * F.x))
-                                         : make_float2((float)(0.5 * F.x), (float)(0.5 * F.y));
-                UB[((size_t)m * cols_pad + col) * Ks + k0 + kl] = u;
-            }
-        };
-        sfft::batch_fft<N1, N2>(nk, getf, put, buf, tw);
-        auto getc = [&](int kl, int n) { return make_double2((double)c2[kl * P + (n < P ? n : n - P)], 0.0); };
-        auto putc = [&](int kl, int m, double2 F) {
-            if (!(m & 1) && m <= P) CV[(size_t)col * J * Ks + (size_t)(m >> 1) * Ks + k0 + kl] = make_double2(0.5 * F.x, 0.5 * F.y);
-        };
-        sfft::batch_fft<N1, N2>(nk, getc, putc, buf, tw);
+        R::run(3 * ((nk + 1) / 2), [&](int f, int n) {
+            const int q = f / 3, ch = f - 3 * q, e = 2 * q * P + n;
+            if (ch == 2) return make_double2((double)c2[e], (double)c2[e + P]);
+            const float2 u = b[e], v = b[e + P];
+            return ch ? sfft::d_mul(make_double2((double)u.y, (double)v.y), tn[n]) : make_double2((double)u.x, (double)v.x);
+        }, buf, tp);
+        for (int e = threadIdx.x; e < M * NP; e += blockDim.x) {
+            const int q = e % NP, m = e / NP;
+            if (2 * q >= nk) continue;
+            double2 u, v;
+            R::pair(m, buf + 3 * q * R::ROW, buf + (3 * q + 1) * R::ROW, u, v);
+            float2 *dst = UB + ((size_t)m * cols_pad + col) * Ks + k0 + 2 * q;
+            dst[0] = make_float2((float)u.x, (float)u.y);
+            if (2 * q + 1 < nk) dst[1] = make_float2((float)v.x, (float)v.y);
+        }
+        for (int e = threadIdx.x; e < J * NP; e += blockDim.x) {
+            const int q = e % NP, j = e / NP;
+            if (2 * q >= nk) continue;
+            double2 u, v;
+            const double2 *z = buf + (3 * q + 2) * R::ROW;
+            R::pair(2 * j, z, z, u, v);
+            double2 *dst = CV + ((size_t)col * J + j) * Ks + k0 + 2 * q;
+            dst[0] = u;
+            if (2 * q + 1 < nk) dst[1] = v;
+        }
     }
 }
 
@@ -375,14 +390,11 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_ptcl_fft(
 static int spec_batches(const Geom &g) { return (g.Ks + sfft::KB - 1) / sfft::KB; }
 static int spec_kb_per_block(const Geom &g, int rows) { return rows >= 16 * 148 ? spec_batches(g) : 1; }
 
-template <int N1, int N2> static size_t spec_ref_fft_smem(int)
+// shared memory of a spectra block: the tables, the rows of CH transforms per shell pair, a batch's samples
+template <int P1, int P2> static size_t spec_fft_smem(int ch, size_t sample)
 {
-    return (size_t)N1 * N2 * sizeof(double2) + (size_t)sfft::buf_elems<N1, N2>() * sizeof(double2) +
-           (size_t)sfft::KB * (N1 * N2 / 2) * sizeof(float2);
-}
-template <int N1, int N2> static size_t spec_ptcl_fft_smem(int)
-{
-    return spec_ref_fft_smem<N1, N2>(0) + (size_t)sfft::KB * (N1 * N2 / 2) * sizeof(float);
+    return (size_t)(2 * P1 * P2 + ch * (sfft::KB / 2) * sfft::Rows<P1, P2>::ROW) * sizeof(double2) +
+           (size_t)sfft::KB * P1 * P2 * sample;
 }
 
 // launches of the spectra kernels: the FFT forms for the supported lengths, the direct
@@ -391,14 +403,14 @@ template <int N1, int N2>
 static cudaError_t launch_spec_ref_fft(pftcc_handle *h, const Geom &g, int ns, const float2 *refs, const float *shifts,
                                        int nrs, int rows_pad, float2 *UA)
 {
-    const size_t smem = spec_ref_fft_smem<N1, N2>(0);
+    const size_t smem = spec_fft_smem<N1, N2>(2, sizeof(float2));
     cudaError_t e = smem_limit((const void *)k_spec_ref_fft<N1, N2>, smem);
     if (e != cudaSuccess) return e;
     const int kbpb = spec_kb_per_block(g, rows_pad);
     const dim3 grid(rows_pad, (spec_batches(g) + kbpb - 1) / kbpb);
     PFTCC_LAUNCH(h);
-    k_spec_ref_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, ns, refs, shifts, h->argtransf, h->argtransf1, 0,
-                                                                    nrs, rows_pad, UA, kbpb);
+    k_spec_ref_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, ns, refs, shifts, h->argtransf, h->argtransf1,
+                                                                    h->d_wn, nrs, rows_pad, UA, kbpb);
     return cudaGetLastError();
 }
 
@@ -406,9 +418,9 @@ static cudaError_t launch_spec_ref(pftcc_handle *h, const Geom &g, int ns, const
                                    int nrs, int rows_pad, float2 *UA)
 {
     switch (g.P) {
-    case 64: return launch_spec_ref_fft<16, 8>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
-    case 180: return launch_spec_ref_fft<24, 15>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
-    case 300: return launch_spec_ref_fft<24, 25>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
+    case 64: return launch_spec_ref_fft<8, 8>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
+    case 180: return launch_spec_ref_fft<12, 15>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
+    case 300: return launch_spec_ref_fft<15, 20>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
     default: break;
     }
     const size_t smem = g.N * sizeof(double2) + (size_t)g.Ks * g.P * sizeof(float2);
@@ -424,14 +436,14 @@ template <int N1, int N2>
 static cudaError_t launch_spec_ptcl_fft(pftcc_handle *h, const Geom &g, const float *ctf, const int *perm, int np,
                                         int cols_pad, float2 *UB, double2 *CV, float *sqp)
 {
-    const size_t smem = spec_ptcl_fft_smem<N1, N2>(0);
+    const size_t smem = spec_fft_smem<N1, N2>(3, sizeof(float2) + sizeof(float));
     cudaError_t e = smem_limit((const void *)k_spec_ptcl_fft<N1, N2>, smem);
     if (e != cudaSuccess) return e;
     const int kbpb = spec_kb_per_block(g, cols_pad);
     const dim3 grid(cols_pad, (spec_batches(g) + kbpb - 1) / kbpb);
     PFTCC_LAUNCH(h);
-    k_spec_ptcl_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, h->ptcls, ctf, perm, np, cols_pad, UB, CV, sqp,
-                                                                     h->sqsums, kbpb);
+    k_spec_ptcl_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, h->ptcls, ctf, perm, h->d_wn, np, cols_pad, UB, CV,
+                                                                     sqp, h->sqsums, kbpb);
     return cudaGetLastError();
 }
 
@@ -439,9 +451,9 @@ static cudaError_t launch_spec_ptcl(pftcc_handle *h, const Geom &g, const float 
                                     int cols_pad, float2 *UB, double2 *CV, float *sqp)
 {
     switch (g.P) {
-    case 64: return launch_spec_ptcl_fft<16, 8>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
-    case 180: return launch_spec_ptcl_fft<24, 15>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
-    case 300: return launch_spec_ptcl_fft<24, 25>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
+    case 64: return launch_spec_ptcl_fft<8, 8>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
+    case 180: return launch_spec_ptcl_fft<12, 15>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
+    case 300: return launch_spec_ptcl_fft<15, 20>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
     default: break;
     }
     const size_t smem = g.N * sizeof(double2) + (size_t)g.Ks * g.P * (sizeof(float2) + sizeof(float));
@@ -475,52 +487,53 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_r2(Geom g, const float2 *
     }
 }
 
-// The same |ref|^2 spectra by the FP64 transforms of length N = 2P (spec_fft.cuh): RU(j) is
-// F(2j) / 2 of the transform of |ref|^2 continued periodically over the full circle, as the
-// CTF^2 spectra of k_spec_ptcl_fft.  Block (reference, kb_per_block batches of sfft::KB shells).
-template <int N1, int N2>
+// The same |ref|^2 spectra by the FP64 transforms of length P, two shells in each (spec_fft.cuh).
+// Block (reference, kb_per_block batches of sfft::KB shells).
+template <int P1, int P2>
 __global__ void __launch_bounds__(SPEC_THREADS) k_spec_r2_fft(Geom g, const float2 *__restrict__ refs,
+                                                              const double2 *__restrict__ wn,
                                                               double2 *__restrict__ RU, int kb_per_block)
 {
-    constexpr int N = N1 * N2, P = N / 2, J = P / 2 + 1;
+    using R = sfft::Rows<P1, P2>;
+    constexpr int P = P1 * P2, J = P / 2 + 1, NP = sfft::KB / 2;
     extern __shared__ float4 smem4[];
     const int Ks = g.Ks;
     const int ka = blockIdx.y * kb_per_block * sfft::KB, kz = min(Ks, ka + kb_per_block * sfft::KB);
-    double2 *tw = reinterpret_cast<double2 *>(smem4);                              // [N]
-    double2 *buf = tw + N;
-    double *u2 = reinterpret_cast<double *>(buf + sfft::buf_elems<N1, N2>());      // [KB][P]
+    double2 *tn = reinterpret_cast<double2 *>(smem4), *tp = tn + P;
+    double2 *buf = tp + P;                                                         // [NP] transforms' rows
+    double *u2 = reinterpret_cast<double *>(buf + NP * R::ROW);                    // [KB][P]
     const int r = blockIdx.x;
-    for (int e = threadIdx.x; e < N; e += blockDim.x) {
-        double sn, cs;
-        sincospi(-2.0 * e / N, &sn, &cs);
-        tw[e] = make_double2(cs, sn);
-    }
-    const float2 *R = refs + (size_t)r * g.K * P;
+    spec_tables<P>(wn, tn, tp);
+    const float2 *Rf = refs + (size_t)r * g.K * P;
     for (int k0 = ka; k0 < kz; k0 += sfft::KB) {
         const int nk = min(sfft::KB, kz - k0);
-        for (int e = threadIdx.x; e < nk * P; e += blockDim.x) {   // e = kl P + n
-            const float2 x = R[(size_t)k0 * P + e];
+        for (int e = threadIdx.x; e < ((nk + 1) & ~1) * P; e += blockDim.x) {   // e = kl P + n
+            const float2 x = e < nk * P ? Rf[(size_t)k0 * P + e] : make_float2(0.f, 0.f);
             u2[e] = (double)x.x * x.x + (double)x.y * x.y;
         }
-        auto getc = [&](int kl, int n) { return make_double2(u2[kl * P + (n < P ? n : n - P)], 0.0); };
-        auto putc = [&](int kl, int m, double2 F) {
-            if (!(m & 1) && m <= P) RU[(size_t)r * J * Ks + (size_t)(m >> 1) * Ks + k0 + kl] = make_double2(0.5 * F.x, 0.5 * F.y);
-        };
-        sfft::batch_fft<N1, N2>(nk, getc, putc, buf, tw);
+        R::run((nk + 1) / 2, [&](int f, int n) { return make_double2(u2[2 * f * P + n], u2[(2 * f + 1) * P + n]); }, buf, tp);
+        for (int e = threadIdx.x; e < J * NP; e += blockDim.x) {
+            const int q = e % NP, j = e / NP;
+            if (2 * q >= nk) continue;
+            double2 u, v;
+            R::pair(2 * j, buf + q * R::ROW, buf + q * R::ROW, u, v);
+            double2 *dst = RU + ((size_t)r * J + j) * Ks + k0 + 2 * q;
+            dst[0] = u;
+            if (2 * q + 1 < nk) dst[1] = v;
+        }
     }
 }
 
 template <int N1, int N2> static cudaError_t launch_spec_r2_fft(pftcc_handle *h, const Geom &g, const float2 *refs,
                                                                   double2 *RU)
 {
-    const size_t smem = (size_t)N1 * N2 * sizeof(double2) + (size_t)sfft::buf_elems<N1, N2>() * sizeof(double2) +
-                        (size_t)sfft::KB * (N1 * N2 / 2) * sizeof(double);
+    const size_t smem = spec_fft_smem<N1, N2>(1, sizeof(double));
     cudaError_t e = smem_limit((const void *)k_spec_r2_fft<N1, N2>, smem);
     if (e != cudaSuccess) return e;
     const int kbpb = spec_kb_per_block(g, h->nrefs);
     const dim3 grid(h->nrefs, (spec_batches(g) + kbpb - 1) / kbpb);
     PFTCC_LAUNCH(h);
-    k_spec_r2_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, refs, RU, kbpb);
+    k_spec_r2_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, refs, h->d_wn, RU, kbpb);
     return cudaGetLastError();
 }
 
@@ -528,9 +541,9 @@ template <int N1, int N2> static cudaError_t launch_spec_r2_fft(pftcc_handle *h,
 static cudaError_t launch_spec_r2(pftcc_handle *h, const Geom &g, const float2 *refs, double2 *RU)
 {
     switch (g.P) {
-    case 64: return launch_spec_r2_fft<16, 8>(h, g, refs, RU);
-    case 180: return launch_spec_r2_fft<24, 15>(h, g, refs, RU);
-    case 300: return launch_spec_r2_fft<24, 25>(h, g, refs, RU);
+    case 64: return launch_spec_r2_fft<8, 8>(h, g, refs, RU);
+    case 180: return launch_spec_r2_fft<12, 15>(h, g, refs, RU);
+    case 300: return launch_spec_r2_fft<15, 20>(h, g, refs, RU);
     default: break;
     }
     PFTCC_LAUNCH(h);
@@ -548,8 +561,8 @@ static cudaError_t launch_spec_r2(pftcc_handle *h, const Geom &g, const float2 *
 // groups of four rows exchanged by the shell's low bits, so that the transposing stores (a warp takes 8
 // shells x 4 rows) and the 16-byte reads are free of bank conflicts -- the (re, im) pairs it held before
 // cost 32-way conflicts on the way in and 2-way on the way out, as long as the arithmetic -- and two
-// rows share one f32x2 instruction.  1000 particles x 8100 rows, P = 180, Ks = 39: 17.2 ms before, 11.4
-// now (40 TFLOP/s).
+// rows share one f32x2 instruction.  1000 particles x 8100 rows, P = 180, Ks = 39: 17.2 ms before, 13.1
+// now (35 TFLOP/s).
 constexpr int S1_TILE = 64;
 constexpr int COL_TILE = 128;
 

@@ -1,16 +1,19 @@
-// spec_fft.cuh -- FP64 transforms of length N = N1 * N2 over the angular samples of a
-// batch of shells, for the m-domain spectra of the search (k_search.cu).
+// spec_fft.cuh -- FP64 transforms over the angular samples, for the m-domain spectra of the search
+// (k_search.cu), its re-score (k_stage2.cu) and the exact correlations (k_exact_fft.cu).
 //
 // The spectra are U(m, k) = sum_{n<P} v_m(n, k) w_N^{-mn}, m = 0..P, N = 2P, with v_m the
-// real part of the polar sample a(n, k) for even m and its imaginary part for odd m.  Over
-// the full circle the polar samples continue as f(n) = a(n) for n < P and conj(a(n - P))
-// for P <= n < N, whose length-N DFT F gives U(m) = F(m) / 2 for even m and
-// U(m) = -i F(m) / 2 for odd m (the terms a + conj a = 2 Re a and a - conj a = 2i Im a).
-// F is computed by one Cooley-Tukey split, in FP64 with FP64 twiddles:
-//   pass 1, task (shell, n1): a length-N2 DFT over n2 of f(n1 + N1 n2), times w_N^{-n1 k2},
-//           into buf[shell][k2][n1];
-//   pass 2, task (shell, k2): a length-N1 DFT over n1 of buf[shell][k2][.] -> F(k2 + N2 k1).
-// buf rows are padded to N1 + 1 entries (conflict-free shared-memory access in both passes).
+// real part of the polar sample a(n, k) for even m and its imaginary part for odd m: for m = 2j the
+// length-P DFT of the real parts at j, for m = 2j + 1 that of the imaginary parts times w_N^{-n}.  Two
+// shells k, k' go through one complex transform, Z = DFT(v_k + i v_k'), and come apart by the
+// symmetry of real sequences,
+//   even m:  U_k(2j) = (Z(j) + conj Z(P - j)) / 2,       U_k'(2j) = -i (Z(j) - conj Z(P - j)) / 2,
+//   odd m:   the same with Z(P - 1 - j), as U(-m) = conj U(m) and w_N^{-n} shifts the frequencies by 1/2,
+// so a shell pair costs one length-P transform per parity of m (and one for the squares that the
+// normaliser needs) where a length-N transform per shell had four to eight times the operations.
+// A transform is one Cooley-Tukey split P = P1 P2, in FP64 with FP64 twiddles:
+//   pass 1, task (transform, n1): a length-P2 DFT over n2 of f(n1 + P1 n2), times w_P^{-n1 k2},
+//           into row k2 of the transform's rows [P2][P1 | 1] (odd: conflict-free in both passes);
+//   pass 2, task (transform, k2): a length-P1 DFT over n1 of row k2, in place: F(k2 + P2 k1) at k1.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -103,43 +106,54 @@ template <int STEP> struct DFFT<1, STEP> {
     __device__ static void run(double2 *, const double2 *) {}
 };
 
-// the shells per batch and the shared memory of the batch buffer
+// the shells per batch of the spectra kernels
 constexpr int KB = 8;
-template <int N1, int N2> __host__ __device__ constexpr int buf_elems() { return KB * N2 * (N1 + 1); }
 
-// F for the nk <= KB shells of a batch: getf(kl, n) returns f(n) of batch shell kl as
-// double2, put(kl, m, F) receives F(m) for every m < N (the caller keeps what it needs).  All
-// threads of the block take part; buf holds buf_elems<N1, N2>() double2, tw the w_N^{-e} table.
-// Starts and ends with the block synchronised (the caller's staging is visible; buf is free again).
-template <int N1, int N2, class GetF, class Put>
-__device__ __forceinline__ void batch_fft(int nk, const GetF &getf, const Put &put, double2 *buf, const double2 *tw)
-{
-    __syncthreads();
-    // pass 1: tasks (kl, n1), n1 fastest
-    for (int t = threadIdx.x; t < nk * N1; t += blockDim.x) {
-        const int kl = t / N1, n1 = t - kl * N1;
-        double2 x[N2];
+template <int P1, int P2> struct Rows {
+    static constexpr int P = P1 * P2, RS = P1 | 1, ROW = P2 * RS;   // double2 of one transform's rows
+    __device__ static int at(int j) { return j % P2 * RS + j / P2; }
+
+    // nf transforms: get(f, n) returns f(n) of transform f; their rows at buf + f ROW hold F afterwards, tw
+    // the w_P^{-e} table.  All threads of the block take part; starts and ends with the block synchronised.
+    template <class Get> __device__ static void run(int nf, const Get &get, double2 *buf, const double2 *tw)
+    {
+        __syncthreads();
+        for (int e = threadIdx.x; e < nf * P1; e += blockDim.x) {
+            const int f = e / P1, n1 = e - f * P1;
+            double2 x[P2];
 #pragma unroll
-        for (int n2 = 0; n2 < N2; ++n2) x[n2] = getf(kl, n1 + N1 * n2);
-        DFFT<N2, N1>::run(x, tw);
-        double2 *row = buf + (size_t)kl * N2 * (N1 + 1) + n1;
+            for (int n2 = 0; n2 < P2; ++n2) x[n2] = get(f, n1 + P1 * n2);
+            DFFT<P2, P1>::run(x, tw);
+            double2 *row = buf + (size_t)f * ROW + n1;
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) row[k2 * (N1 + 1)] = (k2 == 0 || n1 == 0) ? x[k2] : d_mul(x[k2], tw[n1 * k2]);
+            for (int k2 = 0; k2 < P2; ++k2) row[k2 * RS] = k2 == 0 ? x[k2] : d_mul(x[k2], tw[n1 * k2]);
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < nf * P2; e += blockDim.x) {
+            double2 *row = buf + (size_t)(e / P2) * ROW + (e % P2) * RS;
+            double2 x[P1];
+#pragma unroll
+            for (int n1 = 0; n1 < P1; ++n1) x[n1] = row[n1];
+            DFFT<P1, P2>::run(x, tw);
+#pragma unroll
+            for (int k1 = 0; k1 < P1; ++k1) row[k1] = x[k1];
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    // pass 2: tasks (kl, k2), kl fastest (consecutive shells store next to each other)
-    for (int t = threadIdx.x; t < nk * N2; t += blockDim.x) {
-        const int k2 = t / nk, kl = t - k2 * nk;
-        const double2 *row = buf + ((size_t)kl * N2 + k2) * (N1 + 1);
-        double2 x[N1];
-#pragma unroll
-        for (int n1 = 0; n1 < N1; ++n1) x[n1] = row[n1];
-        DFFT<N1, N2>::run(x, tw);
-#pragma unroll
-        for (int k1 = 0; k1 < N1; ++k1) put(kl, k2 + N2 * k1, x[k1]);
+
+    // the two shells of a pair at a frequency: z = Z(j), y = Z at its mirror
+    __device__ static double2 first(double2 z, double2 y) { return make_double2(0.5 * (z.x + y.x), 0.5 * (z.y - y.y)); }
+    __device__ static double2 second(double2 z, double2 y) { return make_double2(0.5 * (z.y + y.y), 0.5 * (y.x - z.x)); }
+    // U(m) of the pair's two shells from the rows of its even transform (ze) and odd transform (zo)
+    __device__ static void pair(int m, const double2 *ze, const double2 *zo, double2 &u, double2 &v)
+    {
+        const int j = m >> 1;
+        const double2 *z = (m & 1) ? zo : ze;
+        const double2 a = z[at(j)], b = z[at((m & 1) ? P - 1 - j : j == 0 ? 0 : P - j)];
+        u = first(a, b);
+        v = second(a, b);
     }
-    __syncthreads();
-}
+};
 
 }  // namespace sfft
 }  // namespace pftcc
