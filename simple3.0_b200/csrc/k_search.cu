@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_ptcl(
 // wn: the table w_N^{-e}, e < N.  What bounds these kernels: the latency of the FP64 chains and the block's
 // barriers (60 to 96 KB of rows and samples a block, two blocks an SM).  With one transform of length N a
 // shell before: the references of 100 x 81 rows, P = 180, 2.16 ms, now 1.25; the particles of 5130 at
-// P = 300, 3.70 and 2.26, 1000 at P = 64, 0.063 and 0.053.
+// P = 300, 3.70 and 1.99 (2.26 with a batch's loads one after the other), 1000 at P = 64, 0.063 and 0.053.
 template <int P> __device__ __forceinline__ void spec_tables(const double2 *__restrict__ wn, double2 *tn, double2 *tp)
 {
     for (int e = threadIdx.x; e < P; e += blockDim.x) {
@@ -286,14 +286,17 @@ __global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ref_fft(
         for (int i = 0; i < NPT; ++i) {
             const int n = threadIdx.x + i * SPEC_THREADS;
             if (n >= P) continue;
-            for (int kl = 0; kl < nk; ++kl) {
-                const float2 x = Rf[(size_t)(k0 + kl) * P + n];
+            float2 xs[sfft::KB];   // the batch's loads in flight together
+#pragma unroll
+            for (int kl = 0; kl < sfft::KB; ++kl) xs[kl] = kl < nk ? Rf[(size_t)(k0 + kl) * P + n] : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int kl = 0; kl < sfft::KB; ++kl) {
+                const float2 x = xs[kl];
                 const float fr = (float)pr[i], fi = (float)pi[i];
                 a[kl * P + n] = make_float2(x.x * fr - x.y * fi, x.x * fi + x.y * fr);
                 const double nr = pr[i] * qr[i] - pi[i] * qi[i], ni = pr[i] * qi[i] + pi[i] * qr[i];
                 pr[i] = nr; pi[i] = ni;
             }
-            if (nk & 1) a[nk * P + n] = make_float2(0.f, 0.f);
         }
         R::run(2 * ((nk + 1) / 2), [&](int f, int n) {
             const float2 u = a[(f & ~1) * P + n], v = a[(f | 1) * P + n];
@@ -349,7 +352,8 @@ __global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ptcl_fft(
     if (threadIdx.x == 0 && blockIdx.y == 0) sqp_out[col] = sqsums[slot];
     for (int k0 = ka; k0 < kz; k0 += sfft::KB) {
         const int nk = min(sfft::KB, kz - k0);
-        for (int e = threadIdx.x; e < ((nk + 1) & ~1) * P; e += blockDim.x) {   // e = kl P + n; an odd shell's partner is 0
+#pragma unroll 5
+        for (int e = threadIdx.x; e < sfft::KB * P; e += SPEC_THREADS) {   // e = kl P + n; past the last shell 0
             const bool in = e < nk * P;
             const float c = in ? (C ? C[(size_t)k0 * P + e] : 1.f) : 0.f;
             const float2 q = in ? Q[(size_t)k0 * P + e] : make_float2(0.f, 0.f);
@@ -507,7 +511,8 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_r2_fft(Geom g, const floa
     const float2 *Rf = refs + (size_t)r * g.K * P;
     for (int k0 = ka; k0 < kz; k0 += sfft::KB) {
         const int nk = min(sfft::KB, kz - k0);
-        for (int e = threadIdx.x; e < ((nk + 1) & ~1) * P; e += blockDim.x) {   // e = kl P + n
+#pragma unroll 5
+        for (int e = threadIdx.x; e < sfft::KB * P; e += SPEC_THREADS) {   // e = kl P + n; past the last shell 0
             const float2 x = e < nk * P ? Rf[(size_t)k0 * P + e] : make_float2(0.f, 0.f);
             u2[e] = (double)x.x * x.x + (double)x.y * x.y;
         }
