@@ -242,117 +242,6 @@ template <int STEP> struct PFFT<1, STEP> {
     __device__ static void run(C2 *, const TwTables &) {}
 };
 
-// Pass A, split into the pieces the two halves of a row's transform take: class 0 (its
-// own mirror, X(P) closes it), the class pairs (c, P1 - c) for C0 <= c < C1, and for even
-// P1 the self-mirrored class P1/2.  Outputs, times w_P^{-j1 l2}, go to the row's slab
-// (element stride T).
-template <int P1, int P2, class GetX>
-__device__ __forceinline__ void passA_class0(const GetX &getx, float2 *slab, int T, const TwTables &tw)
-{
-    constexpr int P = P1 * P2;
-    float2 xa[P2 + 1];
-#pragma unroll
-    for (int j2 = 0; j2 < P2; ++j2) xa[j2] = getx(P1 * j2);
-    xa[P2] = getx(P);
-    xa[0].y = 0.f;       // X(0) and X(P) are real
-    xa[P2].y = 0.f;
-    float2 z[P2];
-#pragma unroll
-    for (int j2 = 0; j2 < P2; ++j2) z[j2] = make_z(xa[j2], xa[P2 - j2], tw.wN[P1 * j2]);
-    SFFT<P2, P1>::run(z, tw);
-#pragma unroll
-    for (int l2 = 0; l2 < P2; ++l2) slab[(l2 * P1) * T] = z[l2];
-}
-
-// the class-pair loop runs over a runtime range (one copy of its code for both halves of
-// a row's transform); c * l2 < P1 * P2 for every class and pass-B index, so the twiddle
-// indices need no reduction
-template <int P1, int P2, class GetX>
-__device__ __forceinline__ void passA_pairs(int c0, int c1, const GetX &getx, float2 *slab, int T, const TwTables &tw)
-{
-#pragma unroll 1
-    for (int c = c0; c < c1; ++c) {
-        float2 xa[P2], xb[P2];
-#pragma unroll
-        for (int j2 = 0; j2 < P2; ++j2) {
-            xa[j2] = getx(c + P1 * j2);
-            xb[j2] = getx(P1 - c + P1 * j2);
-        }
-        float2 za[P2], zb[P2];
-#pragma unroll
-        for (int j2 = 0; j2 < P2; ++j2) {
-            za[j2] = make_z(xa[j2], xb[P2 - 1 - j2], tw.wN[c + P1 * j2]);
-            zb[j2] = make_z(xb[j2], xa[P2 - 1 - j2], tw.wN[P1 - c + P1 * j2]);
-        }
-        SFFT<P2, P1>::run(za, tw);
-        SFFT<P2, P1>::run(zb, tw);
-#pragma unroll
-        for (int l2 = 0; l2 < P2; ++l2) {
-            slab[(l2 * P1 + c) * T] = l2 == 0 ? za[l2] : c_mul(za[l2], tw.wP[c * l2]);
-            slab[(l2 * P1 + P1 - c) * T] = l2 == 0 ? zb[l2] : c_mul(zb[l2], tw.wP[(P1 - c) * l2]);
-        }
-    }
-}
-
-template <int P1, int P2, class GetX>
-__device__ __forceinline__ void passA_mid(const GetX &getx, float2 *slab, int T, const TwTables &tw)
-{
-    constexpr int P = P1 * P2;
-    if constexpr ((P1 & 1) == 0) {
-        constexpr int c = P1 / 2;
-        float2 xa[P2];
-#pragma unroll
-        for (int j2 = 0; j2 < P2; ++j2) xa[j2] = getx(c + P1 * j2);
-        float2 z[P2];
-#pragma unroll
-        for (int j2 = 0; j2 < P2; ++j2) z[j2] = make_z(xa[j2], xa[P2 - 1 - j2], tw.wN[c + P1 * j2]);
-        SFFT<P2, P1>::run(z, tw);
-#pragma unroll
-        for (int l2 = 0; l2 < P2; ++l2) slab[(l2 * P1 + c) * T] = l2 == 0 ? z[l2] : c_mul(z[l2], tw.wP[(c * l2) % P]);
-    }
-}
-
-// pass B for l2 in [L0, L1): length-P1 DFTs, correlations, argmax (lowest rotation on ties).
-// EU (the Euclidean objective): dinv(rho) is the additive term, the value scale * v + dinv(rho)
-template <int P1, int P2, class Dinv, bool EU = false>
-__device__ __forceinline__ void passB(int L0, int L1, const float2 *slab, int T, const TwTables &tw, const Dinv &dinv,
-                                      float scale, float *cc_out, float &best, int &brot)
-{
-    constexpr int P = P1 * P2;
-#pragma unroll 1
-    for (int l2 = L0; l2 < L1; ++l2) {
-        float2 v[P1];
-#pragma unroll
-        for (int j1 = 0; j1 < P1; ++j1) v[j1] = slab[(l2 * P1 + j1) * T];
-        SFFT<P1, P2>::run(v, tw);
-#pragma unroll
-        for (int l1 = 0; l1 < P1; ++l1) {
-            const int l = l2 + P2 * l1;
-            const int r0 = 2 * l, r1 = 2 * l + 1;
-            const float c0 = EU ? fmaf(scale, v[l1].x, dinv(r0 < P ? r0 : r0 - P))
-                                : scale * v[l1].x * dinv(r0 < P ? r0 : r0 - P);
-            const float c1 = EU ? fmaf(scale, v[l1].y, dinv(r1 < P ? r1 : r1 - P))
-                                : scale * v[l1].y * dinv(r1 < P ? r1 : r1 - P);
-            if (cc_out) { cc_out[r0] = c0; cc_out[r1] = c1; }
-            if (c0 > best || (c0 == best && r0 < brot)) { best = c0; brot = r0; }
-            if (c1 > best || (c1 == best && r1 < brot)) { best = c1; brot = r1; }
-        }
-    }
-}
-
-// the whole per-triple transform in one thread; getx(j) returns X(j) for j = 0..P;
-// dinv(rot) the normalising factor; slab is this thread's shared-memory slab with
-// element stride T
-template <int P1, int P2, class GetX, class Dinv>
-__device__ __forceinline__ void triple_corr(const GetX &getx, const Dinv &dinv, float2 *slab, int T, const TwTables &tw,
-                                            float scale, float *cc_out, float &best, int &brot)
-{
-    passA_class0<P1, P2>(getx, slab, T, tw);
-    passA_pairs<P1, P2>(1, (P1 + 1) / 2, getx, slab, T, tw);
-    passA_mid<P1, P2>(getx, slab, T, tw);
-    passB<P1, P2>(0, P2, slab, T, tw, dinv, scale, cc_out, best, brot);
-}
-
 // ---------------------------------------------------------------------------------------
 struct S2Fast {
     int nshifts, N, nrs_total, nwaves;
@@ -599,12 +488,16 @@ k_stage2_fast(S2Fast sp, const __grid_constant__ TwTables tw, const S2Wave *__re
 // X(m) = 4 sum_k UA[m][rs][k] conj(UB[m][col][k]) from the FP32 spectra, the FP64
 // normaliser from the |ref|^2 and CTF^2 spectra, the same transform and argmax.  One block
 // per particle, its ntop <= 8 candidates in four phases:
-//   A  Y(c, j) = (wgt_j / P) sum_k conj(RU[r_c][j][k]) CV[col][j][k] in FP64, a thread per (c, j);
+//   A  Y(c, j) = (wgt_j / P) sum_k conj(RU[r_c][j][k]) CV[col][j][k] in FP64, eight lanes per j;
 //   B  D(c, rho) from Y by the length-P/2 FP64 transform of the packed half spectrum (the
 //      normaliser's k_norm_fft, split H1 x H2 = P/2), stored as 1/sqrt(D * sqsum_ptcl);
-//   C  X(c, m) in FP32, a thread per (c, m);
-//   D  the per-triple transform and argmax of each candidate (two threads each, the halves of
-//      triple_corr), then the particle's best (lowest id among equal correlations).
+//   C  X(c, m) in FP32, eight lanes per m;
+//   D  the transforms and maxima, a thread per (candidate, class) and (candidate, block), then the
+//      particle's best (lowest id among equal correlations).
+// What bounds it: the candidates' spectra from L2 (16 B x J Ks + 8 B x M Ks each, 2.3 MB a particle at
+// P = 300, Ks = 59).  5130 particles, P = 300: before, with one candidate's loads in flight at a time and
+// the transforms in one warp, 3.65 ms; now 1.4 (0.72 of 2.07 for 2500 particles; 0.43 of 0.87 for 3000 at
+// P = 180; 0.064 of 0.076 for 1000 at P = 64).  More of the candidates' loads unrolled: 0.77 at P = 300.
 template <int P> struct HalfSplit;
 template <> struct HalfSplit<64> { static constexpr int H1 = 8, H2 = 4; };
 template <> struct HalfSplit<180> { static constexpr int H1 = 10, H2 = 9; };
@@ -612,16 +505,22 @@ template <> struct HalfSplit<300> { static constexpr int H1 = 15, H2 = 10; };
 constexpr int RS_MAX = 8;     // candidates per particle
 constexpr int RS_THREADS = 256;
 
-template <int P1, int P2> __host__ __device__ constexpr size_t rescore_smem_bytes()
-{
-    constexpr int P = P1 * P2, J = P / 2 + 1, H = P / 2;
-    constexpr int H1 = HalfSplit<P>::H1, H2 = HalfSplit<P>::H2;
-    return sizeof(double2) * ((size_t)2 * H + (size_t)RS_MAX * J + (size_t)RS_MAX * H2 * (H1 + 1)) +
-           sizeof(float2) * ((size_t)RS_MAX * (P + 1) + (size_t)P * RS_MAX) + sizeof(float) * (size_t)RS_MAX * P;
-}
+// shared memory: the FP64 tables, one region for Y and its transform's rows (phases A and B) and then X and
+// the transforms' slabs (C and D), the FP32 tables, the factors, the blocks' maxima.  59 KB at P = 300: three
+// blocks on an SM, which is what hides the latency of the candidates' loads (with two, 18 of 24 cycles
+// between a warp's instructions went to it).
+template <int P1, int P2> struct RescoreSmem {
+    static constexpr int P = P1 * P2, J = P / 2 + 1, H = P / 2, M = P + 1, H1 = HalfSplit<P>::H1, H2 = HalfSplit<P>::H2;
+    static constexpr size_t rows = sizeof(double2) * ((size_t)RS_MAX * J + (size_t)RS_MAX * H2 * (H1 + 1));
+    static constexpr size_t slabs = sizeof(float2) * ((size_t)RS_MAX * M + (size_t)RS_MAX * (P | 1));
+    static constexpr size_t region = ((rows > slabs ? rows : slabs) + 15) / 16 * 16;
+    static constexpr size_t bytes = sizeof(double2) * 2 * H + region + sizeof(float2) * 2 * P + sizeof(float) * RS_MAX * P +
+                                    (sizeof(float) + sizeof(int)) * RS_MAX * P2;
+};
 
-template <int P1, int P2, bool EU>
-__global__ void __launch_bounds__(RS_THREADS) k_rescore_md(int ncols, int ntop, int Ks, int N, int nshifts,
+// KL: shells of a lane, 8 KL >= Ks
+template <int P1, int P2, bool EU, int KL>
+__global__ void __launch_bounds__(RS_THREADS, P1 * P2 <= 64 ? 4 : 3) k_rescore_md(int ncols, int ntop, int Ks, int N, int nshifts,
                                                            int has_shifts, const TwTables tw,
                                                            const float2 *__restrict__ UA, int rows_pad,
                                                            const float2 *__restrict__ UB, int cols_pad,
@@ -635,11 +534,16 @@ __global__ void __launch_bounds__(RS_THREADS) k_rescore_md(int ncols, int ntop, 
     extern __shared__ float4 smem4[];
     double2 *tw_h = reinterpret_cast<double2 *>(smem4);            // [H] w_{P/2}^{-e}
     double2 *wp = tw_h + H;                                         // [H] w_P^{+e}
-    double2 *Ys = wp + H;                                           // [RS_MAX][J]
+    unsigned char *region = reinterpret_cast<unsigned char *>(wp + H);
+    double2 *Ys = reinterpret_cast<double2 *>(region);              // [RS_MAX][J]
     double2 *buf = Ys + RS_MAX * J;                                 // [RS_MAX][H2][H1 + 1]
-    float2 *Xs = reinterpret_cast<float2 *>(buf + RS_MAX * H2 * (H1 + 1));   // [RS_MAX][M]
-    float2 *slab = Xs + RS_MAX * M;                                 // [P][RS_MAX]
-    float *Ds = reinterpret_cast<float *>(slab + P * RS_MAX);       // [RS_MAX][P]
+    float2 *Xs = reinterpret_cast<float2 *>(region);                // [RS_MAX][M], after Ys and buf
+    float2 *slab = Xs + RS_MAX * M;                                 // [RS_MAX][P | 1]
+    float2 *wp_s = reinterpret_cast<float2 *>(region + RescoreSmem<P1, P2>::region);   // [P] w_P^{-e}
+    float2 *wn_s = wp_s + P;                                        // [P] w_N^{-e}
+    float *Ds = reinterpret_cast<float *>(wn_s + P);                // [RS_MAX][P]
+    float *pbest = Ds + RS_MAX * P;                                 // [RS_MAX][P2] the blocks' maxima
+    int *prot = reinterpret_cast<int *>(pbest + RS_MAX * P2);       // [RS_MAX][P2] and their rotations
     __shared__ int rs_s[RS_MAX];
     __shared__ float bc_s[RS_MAX];
     __shared__ int bi_s[RS_MAX];
@@ -658,33 +562,50 @@ __global__ void __launch_bounds__(RS_THREADS) k_rescore_md(int ncols, int ntop, 
         sincospi(2.0 * e / P, &sn, &cs);
         wp[e] = make_double2(cs, sn);
     }
+    for (int e = t; e < P; e += blockDim.x) { wp_s[e] = tw.wP[e]; wn_s[e] = tw.wN[e]; }
     __syncthreads();
-    // A: Y, eight lanes per (candidate, j) over the shells (coalesced reads), summed by shuffles;
-    // the loop runs the same trips in every warp so that the shuffles see all lanes
-    const int l8 = t & 7, grp = t >> 3;
-    constexpr int NGRP = RS_THREADS / 8;
-    for (int base = 0; base < nc * J; base += NGRP) {
-        const int e = base + grp;
-        const int c = e / J, j = e - c * J;
-        const int rs = e < nc * J ? rs_s[c] : -1;
-        double yr = 0.0, yi = 0.0;
-        if (rs >= 0) {
-            const double2 *ru = RU + ((size_t)(rs / nshifts) * J + j) * Ks;
-            const double2 *cv = CV + ((size_t)cl * J + j) * Ks;
-            for (int k = l8; k < Ks; k += 8) {
-                const double2 u = ru[k], v = cv[k];
-                yr += u.x * v.x + u.y * v.y;
-                yi += u.x * v.y - u.y * v.x;
-            }
-        }
+    // A: Y, eight lanes per j over the shells (coalesced reads) and CPT candidates, GP at a time: the
+    // particle's spectrum is read once for them and the loads of UA_ GP candidates are in flight together (an
+    // empty candidate reads row 0 and is dropped at the end).  With few shells a lane has few loads: then four
+    // candidates a task, all in flight.  The loop runs the same
+    // trips in every warp so that the shuffles see all lanes
+    constexpr int NGRP = RS_THREADS / 8, CPT = KL <= 3 ? 4 : 8, GP = KL <= 3 ? 4 : 1,
+                  UA_ = KL <= 3 ? 1 : 2, UC = KL <= 3 ? 1 : 4;   // unrolled groups of GP: loads in flight
+    const int l8 = t & 7, grp = t >> 3, nq = (nc + CPT - 1) / CPT;
+    for (int base = 0; base < J * nq; base += NGRP) {
+        const int e = min(base + grp, J * nq - 1), j = e / nq, c0 = CPT * (e - j * nq);
+        double2 v[KL];
+        const double2 *cv = CV + ((size_t)cl * J + j) * Ks;
 #pragma unroll
-        for (int o = 4; o; o >>= 1) {
-            yr += __shfl_xor_sync(0xffffffffu, yr, o);
-            yi += __shfl_xor_sync(0xffffffffu, yi, o);
-        }
-        if (e < nc * J && l8 == 0) {
-            const double wgt = ((j == 0 || 2 * j == P) ? 1.0 : 2.0) / P;
-            Ys[c * J + j] = make_double2(wgt * yr, wgt * yi);
+        for (int i = 0; i < KL; ++i) v[i] = l8 + 8 * i < Ks ? cv[l8 + 8 * i] : make_double2(0.0, 0.0);
+#pragma unroll UA_
+        for (int cg = c0; cg < c0 + CPT; cg += GP) {
+            double yr[GP], yi[GP];
+#pragma unroll
+            for (int u = 0; u < GP; ++u) {
+                const int rs = cg + u < nc ? rs_s[cg + u] : -1;
+                const double2 *ru = RU + ((size_t)(max(rs, 0) / nshifts) * J + j) * Ks;
+                yr[u] = yi[u] = 0.0;
+#pragma unroll
+                for (int i = 0; i < KL; ++i) {
+                    if (l8 + 8 * i >= Ks) continue;
+                    const double2 r = ru[l8 + 8 * i];
+                    yr[u] = fma(r.x, v[i].x, fma(r.y, v[i].y, yr[u]));
+                    yi[u] = fma(r.x, v[i].y, fma(-r.y, v[i].x, yi[u]));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < GP; ++u) {
+#pragma unroll
+                for (int o = 4; o; o >>= 1) {
+                    yr[u] += __shfl_xor_sync(0xffffffffu, yr[u], o);
+                    yi[u] += __shfl_xor_sync(0xffffffffu, yi[u], o);
+                }
+                if (base + grp < J * nq && l8 == u && cg + u < nc) {
+                    const double wgt = ((j == 0 || 2 * j == P) ? 1.0 : 2.0) / P;
+                    Ys[(cg + u) * J + j] = make_double2(wgt * yr[u], wgt * yi[u]);
+                }
+            }
         }
     }
     __syncthreads();
@@ -735,63 +656,96 @@ __global__ void __launch_bounds__(RS_THREADS) k_rescore_md(int ncols, int ntop, 
             }
         }
     }
-    // C: X, eight lanes per (candidate, m) over the shells as in A
+    __syncthreads();   // X takes the place of Y and its rows
+    // C: X, eight lanes per m over the shells as in A
     const size_t pa = (size_t)rows_pad * Ks, pb = (size_t)cols_pad * Ks;
-    for (int base = 0; base < nc * M; base += NGRP) {
-        const int e = base + grp;
-        const int c = e / M, m = e - c * M;
-        const int rs = e < nc * M ? rs_s[c] : -1;
-        float xr = 0.f, xi = 0.f;
-        if (rs >= 0) {
-            const float2 *a = UA + (size_t)rs * Ks + (size_t)m * pa, *b = UB + (size_t)cl * Ks + (size_t)m * pb;
-            for (int k = l8; k < Ks; k += 8) {
-                const float2 av = a[k], bv = b[k];
-                xr = fmaf(av.x, bv.x, fmaf(av.y, bv.y, xr));
-                xi = fmaf(av.y, bv.x, fmaf(-av.x, bv.y, xi));
+    for (int base = 0; base < M * nq; base += NGRP) {
+        const int e = min(base + grp, M * nq - 1), m = e / nq, c0 = CPT * (e - m * nq);
+        float2 v[KL];
+        const float2 *b = UB + (size_t)cl * Ks + (size_t)m * pb;
+#pragma unroll
+        for (int i = 0; i < KL; ++i) v[i] = l8 + 8 * i < Ks ? b[l8 + 8 * i] : make_float2(0.f, 0.f);
+#pragma unroll UC
+        for (int cg = c0; cg < c0 + CPT; cg += GP) {
+            float xr[GP], xi[GP];
+#pragma unroll
+            for (int u = 0; u < GP; ++u) {
+                const int rs = cg + u < nc ? rs_s[cg + u] : -1;
+                const float2 *a = UA + (size_t)max(rs, 0) * Ks + (size_t)m * pa;
+                xr[u] = xi[u] = 0.f;
+#pragma unroll
+                for (int i = 0; i < KL; ++i) {
+                    if (l8 + 8 * i >= Ks) continue;
+                    const float2 r = a[l8 + 8 * i];
+                    xr[u] = fmaf(r.x, v[i].x, fmaf(r.y, v[i].y, xr[u]));
+                    xi[u] = fmaf(r.y, v[i].x, fmaf(-r.x, v[i].y, xi[u]));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < GP; ++u) {
+#pragma unroll
+                for (int o = 4; o; o >>= 1) {
+                    xr[u] += __shfl_xor_sync(0xffffffffu, xr[u], o);
+                    xi[u] += __shfl_xor_sync(0xffffffffu, xi[u], o);
+                }
+                // X(0) and X(P) are real
+                if (base + grp < M * nq && l8 == u && cg + u < nc)
+                    Xs[(cg + u) * M + m] = make_float2(4.f * xr[u], (m == 0 || m == P) ? 0.f : 4.f * xi[u]);
             }
         }
-#pragma unroll
-        for (int o = 4; o; o >>= 1) {
-            xr += __shfl_xor_sync(0xffffffffu, xr, o);
-            xi += __shfl_xor_sync(0xffffffffu, xi, o);
-        }
-        if (e < nc * M && l8 == 0) Xs[c * M + m] = make_float2(4.f * xr, 4.f * xi);
     }
     __syncthreads();
-    // D: transform and argmax per candidate, two lanes of warp 0 per candidate (lanes 2c, 2c + 1):
-    // pass A by classes (class 0 and the first half of the mirror pairs; the rest and the
-    // middle class), pass B by blocks [0, LB) and [LB, P2); the halves' maxima are combined
-    // with the lowest rotation among equal maxima
-    if (t < 32) {
-        constexpr int NPAIR = (P1 + 1) / 2, PM = 1 + (NPAIR - 1) / 2, LB = (P2 + 1) / 2;
-        const int c = t >> 1, half = t & 1;
-        const bool act = c < nc;
-        const int rs = act ? rs_s[c] : -1;
+    // D: the transform, pass A a thread per (candidate, class), pass B per (candidate, block) with the
+    // block's maximum, then the candidates' maxima (the lowest rotation among equals)
+    for (int e = t; e < nc * P1; e += blockDim.x) {
+        const int c = e / P1, j1 = e - c * P1;
+        const float2 *x = Xs + c * M;
+        float2 z[P2];
+#pragma unroll
+        for (int j2 = 0; j2 < P2; ++j2) {
+            const int j = j1 + P1 * j2;
+            z[j2] = make_z(x[j], x[P - j], wn_s[j]);
+        }
+        SFFT<P2, P1>::run(z, tw);
+#pragma unroll
+        for (int l2 = 0; l2 < P2; ++l2) slab[c * (P | 1) + l2 * P1 + j1] = l2 == 0 ? z[l2] : c_mul(z[l2], wp_s[j1 * l2]);
+    }
+    __syncthreads();
+    for (int e = t; e < nc * P2; e += blockDim.x) {
+        const int c = e / P2, l2 = e - c * P2;
+        const float2 *x = slab + c * (P | 1) + l2 * P1;
+        const float *ds = Ds + c * P;
+        const float scale = 1.0f / (2.0f * (float)N);
+        float2 v[P1];
+#pragma unroll
+        for (int j1 = 0; j1 < P1; ++j1) v[j1] = x[j1];
+        SFFT<P1, P2>::run(v, tw);
         float best = -INFINITY;
         int brot = 0;
-        float2 *sl = slab + (act ? c : 0);
-        auto getx = [&](int j) { return Xs[c * M + j]; };
-        auto dinv = [&](int rho) { return Ds[c * P + rho]; };
-        if (rs >= 0) {
-            if (half == 0) {
-                passA_class0<P1, P2>(getx, sl, RS_MAX, tw);
-                passA_pairs<P1, P2>(1, PM, getx, sl, RS_MAX, tw);
-            } else {
-                passA_pairs<P1, P2>(PM, NPAIR, getx, sl, RS_MAX, tw);
-                passA_mid<P1, P2>(getx, sl, RS_MAX, tw);
-            }
+#pragma unroll
+        for (int l1 = 0; l1 < P1; ++l1) {
+            const int r0 = 2 * (l2 + P2 * l1), r1 = r0 + 1;
+            const float d0 = ds[r0 < P ? r0 : r0 - P], d1 = ds[r1 < P ? r1 : r1 - P];
+            const float c0 = EU ? fmaf(scale, v[l1].x, d0) : scale * v[l1].x * d0;
+            const float c1 = EU ? fmaf(scale, v[l1].y, d1) : scale * v[l1].y * d1;
+            if (c0 > best) { best = c0; brot = r0; }     // rotations rise with l1
+            if (c1 > best) { best = c1; brot = r1; }
         }
-        __syncwarp();
-        if (rs >= 0)
-            passB<P1, P2, decltype(dinv), EU>(half ? LB : 0, half ? P2 : LB, sl, RS_MAX, tw, dinv,
-                                              1.0f / (2.0f * (float)N), nullptr, best, brot);
-        const float ob = __shfl_xor_sync(0xffffffffu, best, 1);
-        const int orot = __shfl_xor_sync(0xffffffffu, brot, 1);
-        if (ob > best || (ob == best && orot < brot)) { best = ob; brot = orot; }
-        if (act && half == 0) {
-            bc_s[c] = best;
-            bi_s[c] = rs < 0 ? 0x7fffffff : rs * N + brot;
+        pbest[c * P2 + l2] = best;
+        prot[c * P2 + l2] = brot;
+    }
+    __syncthreads();
+    if (t < nc) {
+        const int rs = rs_s[t];
+        float best = -INFINITY;
+        int brot = 0;
+        for (int l2 = 0; l2 < P2; ++l2) {
+            const float c = pbest[t * P2 + l2];
+            const int r = prot[t * P2 + l2];
+            if (c > best || (c == best && r < brot)) { best = c; brot = r; }
         }
+        bc_s[t] = rs < 0 ? -INFINITY : best;
+        bi_s[t] = rs < 0 ? 0x7fffffff : rs * N + brot;
     }
     __syncthreads();
     if (t == 0) {
@@ -927,12 +881,14 @@ static cudaError_t launch_rs(pftcc_handle *h, int ncols, int ntop, int Ks, int n
     TwTables tw;
     fill_tw(tw, P);
     if (ntop < 1 || ntop > RS_MAX) return cudaErrorInvalidValue;
-    const size_t smem = rescore_smem_bytes<P1, P2>();
-    cudaError_t e = smem_limit((const void *)k_rescore_md<P1, P2, EU>, smem);
+    const size_t smem = RescoreSmem<P1, P2>::bytes;
+    auto k = Ks <= 24 ? k_rescore_md<P1, P2, EU, 3> : Ks <= 40 ? k_rescore_md<P1, P2, EU, 5> : k_rescore_md<P1, P2, EU, 8>;
+    if (Ks > 64) return cudaErrorInvalidValue;
+    cudaError_t e = smem_limit((const void *)k, smem);
     if (e != cudaSuccess) return e;
     PFTCC_LAUNCH(h);
     KTimer kt(h, PFTCC_K_EXACT);
-    k_rescore_md<P1, P2, EU><<<ncols, RS_THREADS, smem, h->stream>>>(
+    k<<<ncols, RS_THREADS, smem, h->stream>>>(
         ncols, ntop, Ks, 2 * P, nshifts, has_shifts, tw, UA, rows_pad, UB, cols_pad, RU, CV, sqp, cand, perm, c0, out);
     return cudaGetLastError();
 }
