@@ -701,14 +701,17 @@ __global__ void k_norm_cvt(int n, int J, int Ks, int n_pad, const double2 *__res
 // (u.y, u.y)(v.y, -v.x), k in increasing order.  Block: one j, NY2_R = 8 references x 512
 // particles, 4 warps; every thread takes the 8 references (their spectra read at one address per
 // warp) and the particles l + 32 q (q < 4) of its warp's 128 (coalesced reads), 32 accumulators.
-// Y[(rl * ncols + cl) * J + j] unscaled (the transform applies the weights wgt_j / P).
+// Y[(rl * J + j) * ncols + cl] unscaled (the transform applies the weights wgt_j / P): a warp stores 256
+// consecutive bytes.  What bounds it: the FP32 pipe and the write of Y (8 B a value).  With the j of a pair
+// next to each other instead, every store left 8 bytes of a 32-byte sector to be filled by another block
+// much later: 500 references x 2000 particles, P = 180, Ks = 39: 1.78 ms before, 1.12 now.
 constexpr int NY2_R = 8, NY2_C = 512, NY2_KC = 8;   // references, particles and shells per chunk of a block
 constexpr size_t NY2_SMEM = 2 * (size_t)NY2_KC * NY2_C * sizeof(float2);
 __global__ void __launch_bounds__(128) k_norm_y2(int Ks, int J, const float2 *__restrict__ RUf, int nrefs_p,
                                                  const float2 *__restrict__ CVf, int cols_pad, int r0, int nr, int c0,
                                                  int ncols, float2 *__restrict__ Y)
 {
-    __shared__ float2 us[64][NY2_R];     // the block's references' spectra at this j, [k][reference]
+    __shared__ float4 us[64][NY2_R];     // the block's references' spectra at this j, [k][reference], (x, x, y, y)
     extern __shared__ float2 cvs[];      // [2][NY2_KC][NY2_C] its particles' spectra, NY2_KC shells per chunk
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rb = blockIdx.y * NY2_R, cb0 = blockIdx.x * NY2_C, cb = cb0 + warp * 128, j = blockIdx.z;
@@ -716,7 +719,8 @@ __global__ void __launch_bounds__(128) k_norm_y2(int Ks, int J, const float2 *__
     const float2 *vr = CVf + (size_t)j * Ks * cols_pad;
     for (int e = threadIdx.x; e < NY2_R * Ks; e += blockDim.x) {   // clamped reads (the stores are masked)
         const int k = e / NY2_R, i = e - k * NY2_R;
-        us[k][i] = __ldg(ur + (size_t)k * nrefs_p + r0 + min(rb + i, nr - 1));
+        const float2 u = __ldg(ur + (size_t)k * nrefs_p + r0 + min(rb + i, nr - 1));
+        us[k][i] = make_float4(u.x, u.x, u.y, u.y);
     }
     // the particles' spectra in chunks of NY2_KC shells by asynchronous 8-byte copies, the next chunk
     // in flight while this one is used (clamped columns; the stores are masked)
@@ -756,8 +760,8 @@ __global__ void __launch_bounds__(128) k_norm_y2(int Ks, int J, const float2 *__
                 }
 #pragma unroll
                 for (int i = 0; i < NY2_R; ++i) {
-                    const float2 u = us[k0 + kk][i];
-                    const float2 ux = make_float2(u.x, u.x), uy = make_float2(u.y, u.y);
+                    const float4 u = us[k0 + kk][i];
+                    const float2 ux = make_float2(u.x, u.y), uy = make_float2(u.z, u.w);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         acc[i][q] = __ffma2_rn(ux, v[q], acc[i][q]);
@@ -773,7 +777,7 @@ __global__ void __launch_bounds__(128) k_norm_y2(int Ks, int J, const float2 *__
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int rl = rb + i, cl = cb + lane + 32 * q;
-            if (rl < nr && cl < ncols) Y[((size_t)rl * ncols + cl) * J + j] = acc[i][q];
+            if (rl < nr && cl < ncols) Y[((size_t)rl * J + j) * ncols + cl] = acc[i][q];
         }
 }
 
@@ -802,7 +806,7 @@ __global__ void __launch_bounds__(256) k_norm(Geom g, const float2 *__restrict__
         __syncthreads();
         for (int it = threadIdx.x; it < nb * J; it += blockDim.x) {
             const int rb = it / J, j = it - rb * J;
-            const float2 a = Yg[((size_t)(rb0 + rb) * ncols + cl) * J + j];
+            const float2 a = Yg[((size_t)(rb0 + rb) * J + j) * ncols + cl];
             const double wgt = ((j == 0 || 2 * j == P) ? 1.0 : 2.0) / P;
             Y[(size_t)rb * Jp + j] = make_double2(wgt * a.x, wgt * a.y);
         }
@@ -867,7 +871,8 @@ __global__ void __launch_bounds__(256) k_norm(Geom g, const float2 *__restrict__
 // (H(0) = Re c_0, H(P/2) = Re c_{P/2}, H(j) = c_j / 2, H(P - j) = conj(c_j) / 2), and
 // z(l) = D(2l) + i D(2l + 1) is the length-P/2 inverse DFT of
 // Zh(j) = [H(j) + H(j + P/2)] + i [H(j) - H(j + P/2)] w_P^{+j}, computed as conj of the
-// forward transform of conj(Zh).  One block per particle column, NB references per batch:
+// forward transform of conj(Zh).  A block takes NORM_CB particle columns (whose Y lie next to each other)
+// and a share of the references (blockIdx.y), NB = NORM_CB x NRB pairs per batch:
 //   pass 1, task (reference, n1): a length-N2 DFT over n2 of conj Zh(n1 + N1 n2), times
 //           w_{P/2}^{-n1 k2}, into buf[reference][k2][n1];
 //   pass 2, task (reference, k2): a length-N1 DFT over n1 -> conj z(k2 + N2 k1).
@@ -880,50 +885,63 @@ template <int P> __device__ __forceinline__ int norm_slot(int l, int b)
     return (l % 25) * 12 + (l % 6) * 2 + b;                       // P = 300: block l mod 25, l1 = l mod 12 and l1 + 6
 }
 
+// A batch's factors meet in shared memory (over the rows, which pass 2 has in registers by then) and go
+// out as 16-byte stores: the lanes of a warp hold rotations that lie apart in stage 2's order.
+// What bounds it: reading Y and writing the factors (800 B a pair at P = 180).  1e6 pairs, P = 180: 1.15
+// ms before (a block per column, 8-byte reads of Y, 4-byte stores of the factors), 0.80 now; 486,000 at
+// P = 300 0.96 in six launches before, 1.07 now (worth it for Y's order: both kernels 3.03 before, 2.9 now).
+constexpr int NORM_CB = 8;
+template <int N1, int N2> struct NormFft {
+    static constexpr int H = N1 * N2, P = 2 * H, J = H + 1;
+    static constexpr int NRB = 256 / N2 / NORM_CB, NB = NORM_CB * NRB;   // at most a task per thread in pass 2
+    static constexpr size_t smem = (size_t)(2 * H + NB * N2 * (N1 + 1)) * sizeof(double2) + (size_t)NB * J * sizeof(float2);
+    static_assert(NB * norm_dlen<P>() * sizeof(float) <= NB * N2 * (N1 + 1) * sizeof(double2), "factors over the rows");
+};
+
 template <int N1, int N2>
-__global__ void __launch_bounds__(256) k_norm_fft(const float2 *__restrict__ Yg, int nr, int c0, int ncols, int dcols,
-                                                  const float *__restrict__ sqp, float *__restrict__ D, double dscale,
-                                                  int eu)
+__global__ void __launch_bounds__(256, 2) k_norm_fft(const float2 *__restrict__ Yg, const double2 *__restrict__ wn, int nr,
+                                                  int per, int c0, int ncols, int dcols, const float *__restrict__ sqp,
+                                                  float *__restrict__ D, double dscale, int eu)
 {
-    constexpr int H = N1 * N2, P = 2 * H, J = H + 1;
-    constexpr int NB = 256 / (N1 > N2 ? N1 : N2);
+    using S = NormFft<N1, N2>;
+    constexpr int H = S::H, P = S::P, J = S::J, NRB = S::NRB, NB = S::NB, dlen = norm_dlen<P>();
     extern __shared__ double2 sd[];
     double2 *tw = sd;                 // [H] w_{P/2}^{-e}
     double2 *wp = tw + H;             // [H] w_P^{+e}
-    double2 *buf = wp + H;            // [NB][N2][N1 + 1]
-    float2 *ys = reinterpret_cast<float2 *>(buf + NB * N2 * (N1 + 1));   // [NB][J] the batch's Y rows
-    const int cl = blockIdx.x;
-    if (cl >= ncols) return;
-    const int col = c0 + cl;
+    double2 *buf = wp + H;            // [NB][N2][N1 + 1], then the batch's factors [NB][dlen]
+    float2 *ys = reinterpret_cast<float2 *>(buf + NB * N2 * (N1 + 1));   // [NB][J] the batch's Y, pair kl = r NORM_CB + c
+    float *ds = reinterpret_cast<float *>(buf);
+    const int cb = blockIdx.x * NORM_CB, nc = min(NORM_CB, ncols - cb);
+    const int r_end = min(nr, ((int)blockIdx.y + 1) * per);
     for (int e = threadIdx.x; e < H; e += blockDim.x) {
-        double sn, cs;
-        sincospi(-2.0 * e / H, &sn, &cs);
-        tw[e] = make_double2(cs, sn);
-        sincospi(2.0 * e / P, &sn, &cs);
-        wp[e] = make_double2(cs, sn);
+        tw[e] = wn[4 * e];
+        const double2 w = wn[2 * e];
+        wp[e] = make_double2(w.x, -w.y);
     }
-    const double sq = (double)sqp[col];
-    constexpr int dlen = norm_dlen<P>();
-    // a batch's Y rows (J values each, coalesced) by asynchronous 8-byte copies: the first batch's
-    // before the loop, every later batch's while the previous batch's pass 2 runs (pass 1 has
+    // a batch's Y by asynchronous 8-byte copies (NORM_CB columns of a j are 64 consecutive bytes): the first
+    // batch's before the loop, every later batch's while the previous batch's pass 2 runs (pass 1 has
     // consumed ys by then)
     auto fetch = [&](int b0) {
-        const int n = min(NB, nr - b0);
-        for (int e = threadIdx.x; e < n * J; e += blockDim.x) {
-            const int kl = e / J, j = e - kl * J;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(ys + e)),
-                         "l"(Yg + ((size_t)(b0 + kl) * ncols + cl) * J + j)
+        const int n = min(NRB, r_end - b0);
+        for (int e = threadIdx.x; e < n * J * NORM_CB; e += blockDim.x) {
+            const int c = e % NORM_CB, rj = e / NORM_CB, r = rj / J, j = rj - r * J;
+            if (c >= nc) continue;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(
+                             ys + (size_t)(r * NORM_CB + c) * J + j)),
+                         "l"(Yg + ((size_t)(b0 + r) * J + j) * ncols + cb + c)
                          : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    fetch(0);
-    for (int rb0 = 0; rb0 < nr; rb0 += NB) {
-        const int nb = min(NB, nr - rb0);
+    const int r_first = blockIdx.y * per;
+    fetch(r_first);
+    for (int rb0 = r_first; rb0 < r_end; rb0 += NRB) {
+        const int nb = min(NRB, r_end - rb0) * NORM_CB;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         for (int t = threadIdx.x; t < nb * N1; t += blockDim.x) {
             const int kl = t / N1, n1 = t - kl * N1;
+            if (kl % NORM_CB >= nc) continue;
             const float2 *y = ys + (size_t)kl * J;
             // Y(j) times wgt_j / P: 1 / P at j = 0 and j = P/2, 2 / P otherwise
             const double w1 = 1.0 / P, w2 = 2.0 / P;
@@ -950,15 +968,20 @@ __global__ void __launch_bounds__(256) k_norm_fft(const float2 *__restrict__ Yg,
                 row[k2 * (N1 + 1)] = (k2 == 0 || n1 == 0) ? x[k2] : sfft::d_mul(x[k2], tw[n1 * k2]);
         }
         __syncthreads();
-        if (rb0 + NB < nr) fetch(rb0 + NB);
-        for (int t = threadIdx.x; t < nb * N2; t += blockDim.x) {
-            const int kl = t / N2, k2 = t - kl * N2;
+        if (rb0 + NRB < r_end) fetch(rb0 + NRB);
+        const int t = threadIdx.x, kl = t / N2, k2 = t - kl * N2;
+        const bool on = t < nb * N2 && kl % NORM_CB < nc;
+        double2 x[N1];
+        if (on) {
             const double2 *row = buf + ((size_t)kl * N2 + k2) * (N1 + 1);
-            double2 x[N1];
 #pragma unroll
             for (int n1 = 0; n1 < N1; ++n1) x[n1] = row[n1];
+        }
+        __syncthreads();
+        if (on) {
             sfft::DFFT<N1, N2>::run(x, tw);
-            float *dst = D + ((size_t)(rb0 + kl) * dcols + cl) * dlen;
+            const double sq = (double)sqp[c0 + cb + kl % NORM_CB];
+            float *dst = ds + (size_t)kl * dlen;
 #pragma unroll
             for (int k1 = 0; k1 < N1; ++k1) {
                 const int l = k2 + N2 * k1;
@@ -976,6 +999,15 @@ __global__ void __launch_bounds__(256) k_norm_fft(const float2 *__restrict__ Yg,
                 }
             }
         }
+        __syncthreads();
+        constexpr int Q = dlen / 4;
+        for (int e = threadIdx.x; e < nb * Q; e += blockDim.x) {
+            const int p = e / Q, o = e - p * Q, c = p % NORM_CB;
+            if (c < nc)
+                reinterpret_cast<float4 *>(D + ((size_t)(rb0 + p / NORM_CB) * dcols + cb + c) * dlen)[o] =
+                    reinterpret_cast<const float4 *>(ds)[e];
+        }
+        __syncthreads();
     }
 }
 
@@ -983,12 +1015,16 @@ template <int N1, int N2>
 static cudaError_t launch_norm_fft(pftcc_handle *h, const float2 *Y, int nr, int c0, int ncols, int dcols,
                                    const float *sqp, float *D, double dscale, int eu)
 {
-    constexpr int H = N1 * N2, NB = 256 / (N1 > N2 ? N1 : N2);
-    if (stage2_fast_dlen(2 * H) != norm_dlen<2 * H>()) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)(2 * H + NB * N2 * (N1 + 1)) * sizeof(double2) + (size_t)NB * (H + 1) * sizeof(float2);
-    cudaError_t e = smem_limit((const void *)k_norm_fft<N1, N2>, smem);
+    using S = NormFft<N1, N2>;
+    if (stage2_fast_dlen(S::P) != norm_dlen<S::P>()) return cudaErrorInvalidValue;
+    cudaError_t e = smem_limit((const void *)k_norm_fft<N1, N2>, S::smem);
     if (e != cudaSuccess) return e;
-    k_norm_fft<N1, N2><<<ncols, 256, smem, h->stream>>>(Y, nr, c0, ncols, dcols, sqp, D, dscale, eu);
+    // the references in shares, until there are about eight blocks for each of the 148 SMs
+    const int nx = (ncols + NORM_CB - 1) / NORM_CB, batches = (nr + S::NRB - 1) / S::NRB;
+    const int ny = std::max(1, std::min(batches, (8 * 148 + nx - 1) / nx));
+    const int per = (batches + ny - 1) / ny * S::NRB;
+    k_norm_fft<N1, N2><<<dim3(nx, (nr + per - 1) / per), 256, S::smem, h->stream>>>(Y, h->d_wn, nr, per, c0, ncols, dcols,
+                                                                                    sqp, D, dscale, eu);
     return cudaGetLastError();
 }
 
