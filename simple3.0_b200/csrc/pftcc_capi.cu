@@ -248,23 +248,18 @@ static float kb_apod(float x)
 
 static int f_nint(float x) { return (int)(x >= 0.f ? floorf(x + 0.5f) : -floorf(-x + 0.5f)); }
 
-static int cyci(int lo, int hi, int i)
-{
-    if (i > hi) return lo + (i - hi) - 1;
-    if (i < lo) return hi - (lo - i) + 1;
-    return i;
-}
-
-// init_polarizer (simple_polarizer.f90:41-92): taps [K][P][9] in the order of
-// reshape(w, wlen) (window index in x fastest), offsets into cmat(box/2+1, box) with
-// the conjugation of get_fcomp2D (simple_image.f90:1894-1907) as a bitwise complement.
+// init_polarizer (simple_polarizer.f90:41-92): taps [9][K][P] in the order of
+// reshape(w, wlen) (window index in x fastest), offsets into the window |k| <= kto + 1,
+// h <= kto + 1 of cmat(box/2+1, box) that k_polarize stages (row k at k + kto + 1, kto + 2
+// entries a row), with the conjugation of get_fcomp2D (simple_image.f90:1894-1907) as a bitwise
+// complement.  kto + 2 <= box/2 (checked by pftcc_new), so no address is cyclic.
 static int build_polarizer(pftcc_handle *h, int griddev)
 {
     if (h->pol_griddev == griddev && h->pol_off) return PFTCC_OK;
     const Geom &g = h->g;
-    const int N = g.N, P = g.P, K = g.K, box = g.box, ld = box / 2 + 1;
-    std::vector<int> off((size_t)K * P * 9);
-    std::vector<float> wt((size_t)K * P * 9);
+    const int N = g.N, P = g.P, K = g.K, KM = g.kto + 1, W = g.kto + 2, npts = K * P;
+    std::vector<int16_t> off((size_t)npts * 9);
+    std::vector<float> wt((size_t)npts * 9);
     for (int ik = 0; ik < K; ++ik)
         for (int i = 0; i < P; ++i) {
             const float lx = h->h_polar[(size_t)ik * 2 * N + i], ly = h->h_polar[(size_t)ik * 2 * N + N + i];
@@ -282,21 +277,19 @@ static int build_polarizer(pftcc_handle *h, int griddev)
             for (int m = 0; m < 3; ++m)
                 for (int l = 0; l < 3; ++l) {
                     const int t = m * 3 + l;
-                    const int hh = cyci(-box / 2, box / 2, w1 + l);
-                    const int kk = cyci(-box / 2, box / 2 - 1, w2 + m);
-                    int p1, p2, conj = 0;
-                    if (hh >= 0) { p1 = hh; p2 = kk + (kk < 0 ? box : 0); }
-                    else { p1 = -hh; p2 = -kk + (-kk < 0 ? box : 0); conj = 1; }
-                    const int o = p2 * ld + p1;
-                    off[((size_t)ik * P + i) * 9 + t] = conj ? ~o : o;
-                    wt[((size_t)ik * P + i) * 9 + t] = griddev ? w[l][m] : w[l][m] / wsum;
+                    const bool conj = w1 + l < 0;
+                    const int hh = conj ? -(w1 + l) : w1 + l, kk = conj ? -(w2 + m) : w2 + m;
+                    const int o = (kk + KM) * W + hh;
+                    const size_t at = (size_t)t * npts + (size_t)ik * P + i;
+                    off[at] = (int16_t)(conj ? ~o : o);
+                    wt[at] = griddev ? w[l][m] : w[l][m] / wsum;
                 }
         }
     if (!h->pol_off) {
-        ST(dev_alloc(h, (void **)&h->pol_off, off.size() * sizeof(int), "gridding offsets"));
+        ST(dev_alloc(h, (void **)&h->pol_off, off.size() * sizeof(int16_t), "gridding offsets"));
         ST(dev_alloc(h, (void **)&h->pol_w, wt.size() * sizeof(float), "gridding weights"));
     }
-    CK(cudaMemcpyAsync(h->pol_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream), "taps");
+    CK(cudaMemcpyAsync(h->pol_off, off.data(), off.size() * sizeof(int16_t), cudaMemcpyHostToDevice, h->stream), "taps");
     CK(cudaMemcpyAsync(h->pol_w, wt.data(), wt.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream), "taps");
     CK(cudaStreamSynchronize(h->stream), "taps");
     h->pol_griddev = griddev;
@@ -809,7 +802,7 @@ int pftcc_create_polar_absctfmats(pftcc_handle *h, const pftcc_ctfparams *params
                        h->stream), "ctf params");
     for (int c0 = 0; c0 < h->nptcls; c0 += 65535) {
         const int n = std::min(65535, h->nptcls - c0);
-        CK(launch_ctfmat(h, h->d_ctfp + c0, n, h->ctfmats + (size_t)c0 * h->g.K * h->g.P, 0.f, 0), "ctfmat");
+        CK(launch_ctfmat(h, h->d_ctfp + c0, n, h->ctfmats + (size_t)c0 * h->g.K * h->g.P), "ctfmat");
     }
     CK(cudaStreamSynchronize(h->stream), "ctfmat");
     h->ctf_ready = 1;

@@ -148,7 +148,7 @@ struct pftcc_handle {
     std::vector<double> h_argtransf, h_argtransf1;
     std::vector<float> angtab;           // degrees
     // polarizer tables
-    int *pol_off = nullptr;
+    int16_t *pol_off = nullptr;          // [9][K P] into the gridding window (k_polarize)
     float *pol_w = nullptr;
     int pol_griddev = -1;
     void *pol_stage = nullptr;           // device staging of host images
@@ -252,8 +252,7 @@ cudaError_t launch_fproject_polar(pftcc_handle *h, int box, const float2 *cube, 
 // dout [n][3][K][P]
 cudaError_t launch_fdf_project_polar(pftcc_handle *h, int box, const float2 *cube, const double *RD, int n,
                                      float2 *out, float2 *dout);
-cudaError_t launch_ctfmat(pftcc_handle *h, const pftcc_ctfparams *params, int n, float *out, float ddf,
-                          int derivative);
+cudaError_t launch_ctfmat(pftcc_handle *h, const pftcc_ctfparams *params, int n, float *out);
 cudaError_t launch_sqsums(pftcc_handle *h, int first_slot, int n);
 // max_items: the most work items any of the groups has.  rotmask (optional) [ngroups][N]: MODE_BEST /
 // MODE_ITEMMAX take their maxima over the rotations whose mask byte is non-zero
