@@ -3,6 +3,8 @@
 // setters/getters and the per-pair and batched correlation entry points.
 #include "pftcc_internal.cuh"
 
+#include <system_error>
+#include <thread>
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -313,6 +315,10 @@ static void free_all(pftcc_handle *h)
     if (own) cudaStreamDestroy(own);
     for (void *&p : h->pin) { if (p) cudaFreeHost(p); p = nullptr; }
     if (h->pin_cc) cudaFreeHost(h->pin_cc);
+    for (int i = 0; i < 2; ++i) {
+        if (h->dl_buf[i]) cudaFreeHost(h->dl_buf[i]);
+        if (h->dl_ev[i]) cudaEventDestroy(h->dl_ev[i]);
+    }
 }
 
 static int alloc_ptcl_arrays(pftcc_handle *h)
@@ -1635,6 +1641,61 @@ int pftcc_calc_roinv_corrmat(pftcc_handle *h, float *corrmat)
     return PFTCC_OK;
 }
 
+}  // extern "C"
+
+// A large result into the caller's pageable memory: pieces through two pinned buffers, the next piece on its
+// way while this one is copied out by a few threads (which also take the page faults of fresh memory side
+// by side).  One pageable copy of 51 MB took 10.7 ms of corr_all's 13.2, this takes 4.5.  Below
+// two pieces the plain copy is as fast.
+constexpr size_t DL_PIECE = 4u << 20;
+constexpr int DL_THREADS = 4;
+
+static void copy_out(char *dst, const char *src, size_t bytes)
+{
+    std::thread th[DL_THREADS - 1];
+    const size_t part = (bytes / DL_THREADS + 4095) & ~size_t(4095);
+    int started = 0;
+    try {
+        for (; started < DL_THREADS - 1 && (started + 1) * part < bytes; ++started) {
+            const size_t o = (started + 1) * part;
+            th[started] = std::thread([=] { std::memcpy(dst + o, src + o, std::min(part, bytes - o)); });
+        }
+    } catch (const std::system_error &) {   // no more threads: the rest here
+    }
+    std::memcpy(dst, src, std::min(part, bytes));
+    const size_t o = (size_t)(started + 1) * part;
+    if (o < bytes) std::memcpy(dst + o, src + o, bytes - o);
+    for (int i = 0; i < started; ++i) th[i].join();
+}
+
+static int download(pftcc_handle *h, void *dst, const void *src_dev, size_t bytes, const char *what)
+{
+    if (bytes < 2 * DL_PIECE) {
+        CK(cudaMemcpyAsync(dst, src_dev, bytes, cudaMemcpyDeviceToHost, h->stream), what);
+        CK(cudaStreamSynchronize(h->stream), what);
+        return PFTCC_OK;
+    }
+    for (int i = 0; i < 2; ++i) {
+        if (!h->dl_buf[i]) CK(cudaMallocHost(&h->dl_buf[i], DL_PIECE), what);
+        if (!h->dl_ev[i]) CK(cudaEventCreateWithFlags(&h->dl_ev[i], cudaEventDisableTiming), what);
+    }
+    const size_t n = (bytes + DL_PIECE - 1) / DL_PIECE;
+    auto size = [&](size_t i) { return std::min(DL_PIECE, bytes - i * DL_PIECE); };
+    for (size_t i = 0; i <= n; ++i) {
+        if (i < n) {   // the buffer was copied out two pieces ago
+            CK(cudaMemcpyAsync(h->dl_buf[i & 1], static_cast<const char *>(src_dev) + i * DL_PIECE, size(i),
+                               cudaMemcpyDeviceToHost, h->stream), what);
+            CK(cudaEventRecord(h->dl_ev[i & 1], h->stream), what);
+        }
+        if (i == 0) continue;
+        CK(cudaEventSynchronize(h->dl_ev[(i - 1) & 1]), what);
+        copy_out(static_cast<char *>(dst) + (i - 1) * DL_PIECE, static_cast<const char *>(h->dl_buf[(i - 1) & 1]), size(i - 1));
+    }
+    return PFTCC_OK;
+}
+
+extern "C" {
+
 int pftcc_corr_all(pftcc_handle *h, int nshifts, const float *shifts, float *cc)
 {
     if (!h || !cc || nshifts < 0 || (nshifts > 0 && !shifts)) return set_err(h, PFTCC_ERR_ARG, "corr_all: bad arguments");
@@ -1667,9 +1728,7 @@ int pftcc_corr_all(pftcc_handle *h, int nshifts, const float *shifts, float *cc)
         CK(cudaMemcpyAsync(h->d_groups, groups.data(), m * sizeof(Group), cudaMemcpyHostToDevice, h->stream), "groups");
         CK(launch_exact(h, h->d_groups, m, h->d_work, h->d_shifts, MODE_FULL, exact_frame(h), 1, (int)per_ptcl, h->d_out, nullptr),
            "corr_all kernel");
-        CK(cudaMemcpyAsync(cc + (size_t)c0 * out_per_ptcl, h->d_out, (size_t)m * out_per_ptcl * sizeof(float),
-                           cudaMemcpyDeviceToHost, h->stream), "corr_all download");
-        CK(cudaStreamSynchronize(h->stream), "corr_all");
+        ST(download(h, cc + (size_t)c0 * out_per_ptcl, h->d_out, (size_t)m * out_per_ptcl * sizeof(float), "corr_all download"));
     }
     return PFTCC_OK;
 }
@@ -1686,9 +1745,7 @@ int pftcc_corr_all_prec(pftcc_handle *h, int nshifts, const float *shifts, int p
     const size_t n = (size_t)h->nptcls * h->nrefs * std::max(1, nshifts) * h->g.N;
     ST(ensure(h, (void **)&h->d_out, &h->out_cap, n * sizeof(float), "corr_all_prec out"));
     ST(search_mdomain(h, nshifts, shifts, precision, 0, nullptr, h->d_out));
-    CK(cudaMemcpyAsync(cc, h->d_out, n * sizeof(float), cudaMemcpyDeviceToHost, h->stream), "corr_all_prec download");
-    CK(cudaStreamSynchronize(h->stream), "corr_all_prec");
-    return PFTCC_OK;
+    return download(h, cc, h->d_out, n * sizeof(float), "corr_all_prec download");
 }
 
 static int search_exact(pftcc_handle *h, int nshifts, const float *shifts, pftcc_best *out_dev)

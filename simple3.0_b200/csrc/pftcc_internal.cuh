@@ -189,6 +189,9 @@ struct pftcc_handle {
     float *pin_cc = nullptr;             // [N] pinned: one gencorrs call's result, written by its kernel
     pftcc_best *d_best = nullptr;
     size_t best_cap = 0;
+    // the pinned pieces of a large download and their events
+    void *dl_buf[2] = {nullptr, nullptr};
+    cudaEvent_t dl_ev[2] = {nullptr, nullptr};
     pftcc::SearchWS ws;
     std::mutex mtx;
     std::string last_err;
