@@ -704,15 +704,17 @@ __global__ void k_norm_cvt(int n, int J, int Ks, int n_pad, const double2 *__res
 // Y[(rl * J + j) * ncols + cl] unscaled (the transform applies the weights wgt_j / P): a warp stores 256
 // consecutive bytes.  What bounds it: the FP32 pipe and the write of Y (8 B a value).  With the j of a pair
 // next to each other instead, every store left 8 bytes of a 32-byte sector to be filled by another block
-// much later: 500 references x 2000 particles, P = 180, Ks = 39: 1.78 ms before, 1.12 now.
+// much later: 500 references x 2000 particles, P = 180, Ks = 39: 1.78 ms before, 0.98 now (29 TFLOP/s).
 constexpr int NY2_R = 8, NY2_C = 512, NY2_KC = 8;   // references, particles and shells per chunk of a block
-constexpr size_t NY2_SMEM = 2 * (size_t)NY2_KC * NY2_C * sizeof(float2);
+constexpr int NY2_CS = NY2_C + 2;                    // a chunk's row: from an even column (16-byte copies)
+constexpr size_t NY2_SMEM = 2 * (size_t)NY2_KC * NY2_CS * sizeof(float2);
 __global__ void __launch_bounds__(128) k_norm_y2(int Ks, int J, const float2 *__restrict__ RUf, int nrefs_p,
                                                  const float2 *__restrict__ CVf, int cols_pad, int r0, int nr, int c0,
                                                  int ncols, float2 *__restrict__ Y)
 {
     __shared__ float4 us[64][NY2_R];     // the block's references' spectra at this j, [k][reference], (x, x, y, y)
-    extern __shared__ float2 cvs[];      // [2][NY2_KC][NY2_C] its particles' spectra, NY2_KC shells per chunk
+    extern __shared__ float4 smem4[];
+    float2 *cvs = reinterpret_cast<float2 *>(smem4);   // [2][NY2_KC][NY2_CS] its particles' spectra, NY2_KC shells per chunk
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rb = blockIdx.y * NY2_R, cb0 = blockIdx.x * NY2_C, cb = cb0 + warp * 128, j = blockIdx.z;
     const float2 *ur = RUf + (size_t)j * Ks * nrefs_p;
@@ -722,18 +724,22 @@ __global__ void __launch_bounds__(128) k_norm_y2(int Ks, int J, const float2 *__
         const float2 u = __ldg(ur + (size_t)k * nrefs_p + r0 + min(rb + i, nr - 1));
         us[k][i] = make_float4(u.x, u.x, u.y, u.y);
     }
-    // the particles' spectra in chunks of NY2_KC shells by asynchronous 8-byte copies, the next chunk
-    // in flight while this one is used (clamped columns; the stores are masked)
+    // the particles' spectra in chunks of NY2_KC shells by asynchronous 16-byte copies of column pairs, the next
+    // chunk in flight while this one is used; the row starts at the even column at or before the block's
+    // first, and pairs past the padded columns are left out (the stores are masked).  8-byte copies with an
+    // index division each were a third of the kernel's instructions
     const int nch = (Ks + NY2_KC - 1) / NY2_KC;
+    const int ce = (c0 + cb0) & ~1, odd = (c0 + cb0) & 1, np = min(NY2_CS, cols_pad - ce) / 2;   // cols_pad is even
     auto fetch = [&](int ch) {
-        float2 *dst = cvs + (size_t)(ch & 1) * NY2_KC * NY2_C;
+        float2 *dst = cvs + (size_t)(ch & 1) * NY2_KC * NY2_CS;
         const int k0 = ch * NY2_KC, nk = min(NY2_KC, Ks - k0);
-        for (int e = threadIdx.x; e < nk * NY2_C; e += blockDim.x) {
-            const int kk = e / NY2_C, c = e - kk * NY2_C;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + e)),
-                         "l"(vr + (size_t)(k0 + kk) * cols_pad + c0 + min(cb0 + c, ncols - 1))
-                         : "memory");
-        }
+        const float2 *src = vr + (size_t)k0 * cols_pad + ce;
+        for (int kk = 0; kk < nk; ++kk)
+            for (int p = threadIdx.x; p < np; p += 128)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(
+                                 dst + kk * NY2_CS + 2 * p)),
+                             "l"(src + (size_t)kk * cols_pad + 2 * p)
+                             : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     fetch(0);
@@ -747,7 +753,7 @@ __global__ void __launch_bounds__(128) k_norm_y2(int Ks, int J, const float2 *__
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();    // chunk ch landed for everyone; chunk ch - 1's buffer is free
         if (ch + 1 < nch) fetch(ch + 1);
-        const float2 *cv = cvs + (size_t)(ch & 1) * NY2_KC * NY2_C + warp * 128 + lane;
+        const float2 *cv = cvs + (size_t)(ch & 1) * NY2_KC * NY2_CS + odd + warp * 128 + lane;
         const int k0 = ch * NY2_KC, nk = min(NY2_KC, Ks - k0);
         if (active) {
 #pragma unroll 4
@@ -755,7 +761,7 @@ __global__ void __launch_bounds__(128) k_norm_y2(int Ks, int J, const float2 *__
                 float2 v[4], vb[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    v[q] = cv[kk * NY2_C + 32 * q];
+                    v[q] = cv[kk * NY2_CS + 32 * q];
                     vb[q] = make_float2(v[q].y, -v[q].x);
                 }
 #pragma unroll
