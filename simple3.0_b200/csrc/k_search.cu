@@ -225,9 +225,13 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_ptcl(
 // single-precision shift phases of the de Moivre recurrence), a batch of shells at a time
 // ([shell][n] in shared memory), the recurrence state kept per angular sample n.
 // wn: the table w_N^{-e}, e < N.  What bounds these kernels: the latency of the FP64 chains and the block's
-// barriers (60 to 96 KB of rows and samples a block, two blocks an SM).  With one transform of length N a
-// shell before: the references of 100 x 81 rows, P = 180, 2.16 ms, now 1.25; the particles of 5130 at
-// P = 300, 3.70 and 1.99 (2.26 with a batch's loads one after the other), 1000 at P = 64, 0.063 and 0.053.
+// barriers, with 40 to 96 KB of rows and samples a block.  T threads: about the larger pass's tasks of a batch
+// (a thread per transform and P1 or P2, two transforms a shell pair for the references, three for the particles,
+// one for |ref|^2, four pairs), so that small blocks share an SM instead of idle warps meeting at the barriers;
+// the particles' blocks, two an SM by their memory, stay at 256 from P = 180 on (192 threads: 0.70 ms, not 0.64).
+// With one transform of length N a shell before: the references of 100 x 81 rows, P = 180, 2.16 ms, then 1.23
+// with 256 threads, now 0.97 (P = 64, 100 x 25 rows: 0.17 and 0.10); the particles of 5130 at P = 300, 3.70 and
+// 1.99 (2.26 with a batch's loads one after the other), 1000 at P = 64, 0.063 and 0.048.
 template <int P> __device__ __forceinline__ void spec_tables(const double2 *__restrict__ wn, double2 *tn, double2 *tp)
 {
     for (int e = threadIdx.x; e < P; e += blockDim.x) {
@@ -236,14 +240,14 @@ template <int P> __device__ __forceinline__ void spec_tables(const double2 *__re
     }
 }
 
-template <int P1, int P2>
-__global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ref_fft(
+template <int P1, int P2, int T>
+__global__ void __launch_bounds__(T, 512 / T) k_spec_ref_fft(
     Geom g, int nshifts, const float2 *__restrict__ refs, const float *__restrict__ shifts,
     const double *__restrict__ argtransf, const double *__restrict__ argtransf1, const double2 *__restrict__ wn, int nrs,
     int rows_pad, float2 *__restrict__ UA, int kb_per_block)
 {
     using R = sfft::Rows<P1, P2>;
-    constexpr int P = P1 * P2, NPT = (P + SPEC_THREADS - 1) / SPEC_THREADS, NP = sfft::KB / 2;
+    constexpr int P = P1 * P2, NPT = (P + T - 1) / T, NP = sfft::KB / 2;
     extern __shared__ float4 smem4[];
     const int Ks = g.Ks, M = P + 1;
     // this block's shells [ka, kz): blockIdx.y selects kb_per_block batches of sfft::KB
@@ -268,7 +272,7 @@ __global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ref_fft(
     double pr[NPT], pi[NPT], qr[NPT], qi[NPT];
 #pragma unroll
     for (int i = 0; i < NPT; ++i) {
-        const int n = threadIdx.x + i * SPEC_THREADS;
+        const int n = threadIdx.x + i * T;
         pr[i] = 1.0; pi[i] = 0.0; qr[i] = 1.0; qi[i] = 0.0;
         if (n < P) {
             sincos(argtransf[n] * sx + argtransf[P + n] * sy, &pi[i], &pr[i]);
@@ -284,7 +288,7 @@ __global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ref_fft(
         const int nk = min(sfft::KB, kz - k0);
 #pragma unroll
         for (int i = 0; i < NPT; ++i) {
-            const int n = threadIdx.x + i * SPEC_THREADS;
+            const int n = threadIdx.x + i * T;
             if (n >= P) continue;
             float2 xs[sfft::KB];   // the batch's loads in flight together
 #pragma unroll
@@ -316,8 +320,8 @@ __global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ref_fft(
 
 // particle-side spectra by the FP64 transforms: UB[m][col][k] of B = |CTF| * ptcl and the
 // CTF^2 spectra CV[col][j][k] = sum_{n<P} CTF^2(n, k) w_P^{-jn}, a third transform per shell pair
-template <int P1, int P2>
-__global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ptcl_fft(
+template <int P1, int P2, int T>
+__global__ void __launch_bounds__(T, 512 / T) k_spec_ptcl_fft(
     Geom g, const float2 *__restrict__ ptcls, const float *__restrict__ ctfmats, const int *__restrict__ perm,
     const double2 *__restrict__ wn, int ncols, int cols_pad, float2 *__restrict__ UB, double2 *__restrict__ CV,
     float *__restrict__ sqp_out, const float *__restrict__ sqsums, int kb_per_block)
@@ -353,7 +357,7 @@ __global__ void __launch_bounds__(SPEC_THREADS, 2) k_spec_ptcl_fft(
     for (int k0 = ka; k0 < kz; k0 += sfft::KB) {
         const int nk = min(sfft::KB, kz - k0);
 #pragma unroll 5
-        for (int e = threadIdx.x; e < sfft::KB * P; e += SPEC_THREADS) {   // e = kl P + n; past the last shell 0
+        for (int e = threadIdx.x; e < sfft::KB * P; e += T) {   // e = kl P + n; past the last shell 0
             const bool in = e < nk * P;
             const float c = in ? (C ? C[(size_t)k0 * P + e] : 1.f) : 0.f;
             const float2 q = in ? Q[(size_t)k0 * P + e] : make_float2(0.f, 0.f);
@@ -403,17 +407,17 @@ template <int P1, int P2> static size_t spec_fft_smem(int ch, size_t sample)
 
 // launches of the spectra kernels: the FFT forms for the supported lengths, the direct
 // sums otherwise (identical spectra up to FP64 rounding before the final FP32 / FP64 store)
-template <int N1, int N2>
+template <int N1, int N2, int T>
 static cudaError_t launch_spec_ref_fft(pftcc_handle *h, const Geom &g, int ns, const float2 *refs, const float *shifts,
                                        int nrs, int rows_pad, float2 *UA)
 {
     const size_t smem = spec_fft_smem<N1, N2>(2, sizeof(float2));
-    cudaError_t e = smem_limit((const void *)k_spec_ref_fft<N1, N2>, smem);
+    cudaError_t e = smem_limit((const void *)k_spec_ref_fft<N1, N2, T>, smem);
     if (e != cudaSuccess) return e;
     const int kbpb = spec_kb_per_block(g, rows_pad);
     const dim3 grid(rows_pad, (spec_batches(g) + kbpb - 1) / kbpb);
     PFTCC_LAUNCH(h);
-    k_spec_ref_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, ns, refs, shifts, h->argtransf, h->argtransf1,
+    k_spec_ref_fft<N1, N2, T><<<grid, T, smem, h->stream>>>(g, ns, refs, shifts, h->argtransf, h->argtransf1,
                                                                     h->d_wn, nrs, rows_pad, UA, kbpb);
     return cudaGetLastError();
 }
@@ -422,9 +426,9 @@ static cudaError_t launch_spec_ref(pftcc_handle *h, const Geom &g, int ns, const
                                    int nrs, int rows_pad, float2 *UA)
 {
     switch (g.P) {
-    case 64: return launch_spec_ref_fft<8, 8>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
-    case 180: return launch_spec_ref_fft<12, 15>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
-    case 300: return launch_spec_ref_fft<15, 20>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
+    case 64: return launch_spec_ref_fft<8, 8, 64>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
+    case 180: return launch_spec_ref_fft<12, 15, 128>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
+    case 300: return launch_spec_ref_fft<15, 20, 160>(h, g, ns, refs, shifts, nrs, rows_pad, UA);
     default: break;
     }
     const size_t smem = g.N * sizeof(double2) + (size_t)g.Ks * g.P * sizeof(float2);
@@ -436,17 +440,17 @@ static cudaError_t launch_spec_ref(pftcc_handle *h, const Geom &g, int ns, const
     return cudaGetLastError();
 }
 
-template <int N1, int N2>
+template <int N1, int N2, int T>
 static cudaError_t launch_spec_ptcl_fft(pftcc_handle *h, const Geom &g, const float *ctf, const int *perm, int np,
                                         int cols_pad, float2 *UB, double2 *CV, float *sqp)
 {
     const size_t smem = spec_fft_smem<N1, N2>(3, sizeof(float2) + sizeof(float));
-    cudaError_t e = smem_limit((const void *)k_spec_ptcl_fft<N1, N2>, smem);
+    cudaError_t e = smem_limit((const void *)k_spec_ptcl_fft<N1, N2, T>, smem);
     if (e != cudaSuccess) return e;
     const int kbpb = spec_kb_per_block(g, cols_pad);
     const dim3 grid(cols_pad, (spec_batches(g) + kbpb - 1) / kbpb);
     PFTCC_LAUNCH(h);
-    k_spec_ptcl_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, h->ptcls, ctf, perm, h->d_wn, np, cols_pad, UB, CV,
+    k_spec_ptcl_fft<N1, N2, T><<<grid, T, smem, h->stream>>>(g, h->ptcls, ctf, perm, h->d_wn, np, cols_pad, UB, CV,
                                                                      sqp, h->sqsums, kbpb);
     return cudaGetLastError();
 }
@@ -455,9 +459,9 @@ static cudaError_t launch_spec_ptcl(pftcc_handle *h, const Geom &g, const float 
                                     int cols_pad, float2 *UB, double2 *CV, float *sqp)
 {
     switch (g.P) {
-    case 64: return launch_spec_ptcl_fft<8, 8>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
-    case 180: return launch_spec_ptcl_fft<12, 15>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
-    case 300: return launch_spec_ptcl_fft<15, 20>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
+    case 64: return launch_spec_ptcl_fft<8, 8, 96>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
+    case 180: return launch_spec_ptcl_fft<12, 15, 256>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
+    case 300: return launch_spec_ptcl_fft<15, 20, 256>(h, g, ctf, perm, np, cols_pad, UB, CV, sqp);
     default: break;
     }
     const size_t smem = g.N * sizeof(double2) + (size_t)g.Ks * g.P * (sizeof(float2) + sizeof(float));
@@ -493,10 +497,9 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_r2(Geom g, const float2 *
 
 // The same |ref|^2 spectra by the FP64 transforms of length P, two shells in each (spec_fft.cuh).
 // Block (reference, kb_per_block batches of sfft::KB shells).
-template <int P1, int P2>
-__global__ void __launch_bounds__(SPEC_THREADS) k_spec_r2_fft(Geom g, const float2 *__restrict__ refs,
-                                                              const double2 *__restrict__ wn,
-                                                              double2 *__restrict__ RU, int kb_per_block)
+template <int P1, int P2, int T>
+__global__ void __launch_bounds__(T) k_spec_r2_fft(Geom g, const float2 *__restrict__ refs, const double2 *__restrict__ wn,
+                                                   double2 *__restrict__ RU, int kb_per_block)
 {
     using R = sfft::Rows<P1, P2>;
     constexpr int P = P1 * P2, J = P / 2 + 1, NP = sfft::KB / 2;
@@ -512,7 +515,7 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_r2_fft(Geom g, const floa
     for (int k0 = ka; k0 < kz; k0 += sfft::KB) {
         const int nk = min(sfft::KB, kz - k0);
 #pragma unroll 5
-        for (int e = threadIdx.x; e < sfft::KB * P; e += SPEC_THREADS) {   // e = kl P + n; past the last shell 0
+        for (int e = threadIdx.x; e < sfft::KB * P; e += T) {   // e = kl P + n; past the last shell 0
             const float2 x = e < nk * P ? Rf[(size_t)k0 * P + e] : make_float2(0.f, 0.f);
             u2[e] = (double)x.x * x.x + (double)x.y * x.y;
         }
@@ -529,16 +532,16 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_r2_fft(Geom g, const floa
     }
 }
 
-template <int N1, int N2> static cudaError_t launch_spec_r2_fft(pftcc_handle *h, const Geom &g, const float2 *refs,
-                                                                  double2 *RU)
+template <int N1, int N2, int T>
+static cudaError_t launch_spec_r2_fft(pftcc_handle *h, const Geom &g, const float2 *refs, double2 *RU)
 {
     const size_t smem = spec_fft_smem<N1, N2>(1, sizeof(double));
-    cudaError_t e = smem_limit((const void *)k_spec_r2_fft<N1, N2>, smem);
+    cudaError_t e = smem_limit((const void *)k_spec_r2_fft<N1, N2, T>, smem);
     if (e != cudaSuccess) return e;
     const int kbpb = spec_kb_per_block(g, h->nrefs);
     const dim3 grid(h->nrefs, (spec_batches(g) + kbpb - 1) / kbpb);
     PFTCC_LAUNCH(h);
-    k_spec_r2_fft<N1, N2><<<grid, SPEC_THREADS, smem, h->stream>>>(g, refs, h->d_wn, RU, kbpb);
+    k_spec_r2_fft<N1, N2, T><<<grid, T, smem, h->stream>>>(g, refs, h->d_wn, RU, kbpb);
     return cudaGetLastError();
 }
 
@@ -546,9 +549,9 @@ template <int N1, int N2> static cudaError_t launch_spec_r2_fft(pftcc_handle *h,
 static cudaError_t launch_spec_r2(pftcc_handle *h, const Geom &g, const float2 *refs, double2 *RU)
 {
     switch (g.P) {
-    case 64: return launch_spec_r2_fft<8, 8>(h, g, refs, RU);
-    case 180: return launch_spec_r2_fft<12, 15>(h, g, refs, RU);
-    case 300: return launch_spec_r2_fft<15, 20>(h, g, refs, RU);
+    case 64: return launch_spec_r2_fft<8, 8, 64>(h, g, refs, RU);
+    case 180: return launch_spec_r2_fft<12, 15, 64>(h, g, refs, RU);
+    case 300: return launch_spec_r2_fft<15, 20, 96>(h, g, refs, RU);
     default: break;
     }
     PFTCC_LAUNCH(h);
