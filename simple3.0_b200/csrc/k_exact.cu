@@ -744,16 +744,18 @@ __device__ __forceinline__ RotCtf rot_ctf(const pftcc_ctfparams &p, double ddf)
     return r;
 }
 
-constexpr int FR_MAX = 384;           // k_adjoint's largest block
+constexpr int FR_MAX = 192;           // k_adjoint's largest block
 
-// The block: segments of ceil32(P) threads, thread per n, each segment a share of the shells (two at
-// P = 180, six at 64): every warp is full but the last of a segment, and a single request has the most
-// threads its samples allow.  What bounds it: the FP64 pipe -- about 30 operations a sample and the
-// sine and cosine of the CTF (CTF false: none).
-// 22,000 requests at P = 180, Ks = 39 (recomputed CTF): before, with the arctangent, cosine and optics
-// constants in the loop, seven block sums and 180 of 256 threads, 7.8 ms; now 2.2.
+// The block: segments of tp threads, thread per n (the n in equal steps of whole warps where P passes the
+// block: two of 160 at P = 300), each segment a share of the shells (one at P = 180, three at 64).  What
+// bounds it: the latency of the FP64 chains -- about 30 operations a sample and the sine and cosine of the
+// CTF (CTF false: none) -- so the registers are held to 80 and the blocks kept small: four share an SM.
+// 22,000 requests at P = 180, Ks = 39 (recomputed CTF): 7.8 ms with the arctangent, cosine and optics constants
+// in the loop, seven block sums and 180 of 256 threads; 2.23 with two segments a block of 384 threads and as many
+// registers as it takes, one block an SM (1.48 held to 80 registers); now 1.26 (P = 64: 0.76 and 0.29; 10,000 at
+// P = 300: 1.58 and 1.52).
 template <bool CTF>
-__global__ void __launch_bounds__(FR_MAX) k_adjoint(
+__global__ void __launch_bounds__(FR_MAX, 4) k_adjoint(
     Geom g, int tp, const RotReq *__restrict__ reqs, const RotCtf *__restrict__ rctf, const float2 *__restrict__ refs_even,
     const float2 *__restrict__ refs_odd, const float2 *__restrict__ ptcls, const uint8_t *__restrict__ iseven, const float *__restrict__ polar,
     const double *__restrict__ argtransf, const double *__restrict__ argtransf1, int match_filt,
@@ -844,7 +846,8 @@ __global__ void __launch_bounds__(FR_MAX) k_adjoint(
 static cudaError_t launch_adjoint(pftcc_handle *h, const RotReq *reqs, const RotCtf *rctf, int n, int match_filt,
                                     double *out5)
 {
-    const int tp = std::min(FR_MAX, (h->g.P + 31) / 32 * 32), nseg = std::max(1, std::min(FR_MAX / tp, h->g.Ks));
+    const int steps = (h->g.P + FR_MAX - 1) / FR_MAX, tp = ((h->g.P + steps - 1) / steps + 31) / 32 * 32;
+    const int nseg = std::max(1, std::min(FR_MAX / tp, h->g.Ks));
     auto k = h->cfg.with_ctf && h->ctf_ready ? k_adjoint<true> : k_adjoint<false>;
     PFTCC_LAUNCH(h);
     k<<<n, nseg * tp, 0, h->stream>>>(h->g, tp, reqs, rctf, h->refs_even, h->refs_odd, h->ptcls, h->d_iseven,
