@@ -215,10 +215,10 @@ def algorithmic_costs(w, nshifts, kernel):
 
 
 # DRAM bytes (read + write) per (reference, shift, particle) triple measured by ncu on one
-# launch of the same kernel (box 128 / nrots 360: 4096 rows x 512 columns, 3.0601 GB read +
-# 0.0043 GB written = 1461.2 B per triple against 1440 B algorithmic); the stage-2 traffic grows
+# launch of the same kernel (box 128 / nrots 360: 4096 rows x 512 columns, 3.0409 GB read +
+# 0.0066 GB written = 1453.2 B per triple against 1440 B algorithmic); the stage-2 traffic grows
 # with the triples processed, so the bench scales it to its own launches
-DRAM_BYTES_PER_TRIPLE = {("stage2", 180): (3.060076e9 + 0.004345e9) / (4096 * 512)}
+DRAM_BYTES_PER_TRIPLE = {("stage2", 180): (3.040940e9 + 0.006600e9) / (4096 * 512)}
 
 
 def run_ours(args):
