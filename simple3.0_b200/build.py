@@ -22,7 +22,7 @@ def sources():
 
 
 def _deps():
-    return sources() + sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + [
+    return sources() + sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h"))) + [
         os.path.join(HERE, "..", "include", "pftcc_b200.h"), os.path.abspath(__file__)]
 
 

@@ -31,6 +31,7 @@
 //   k_finish      top-1, or the exact FP32 re-score of the top-ntop (ref, shift)
 #include "pftcc_internal.cuh"
 #include "spec_fft.cuh"
+#include "group_waves.h"
 
 #include <algorithm>
 #include <cmath>
@@ -1549,8 +1550,8 @@ __global__ void k_best_clear(pftcc_best *out, int n)
 // whose spectra, packed operands and candidates are formed per batch, so that the workspace scales
 // with the batch and not with the queue.  Each (parity, group) block of columns against its group's
 // (reference, shift) rows is one wave, cut into several where its packed spectrum would pass the
-// per-wave budget; the waves of a batch run as ONE persistent tcgen05 stage-1 launch over all their
-// work items (the device wave table, umma_stage1_waves), the normaliser per wave, and ONE stage-2
+// per-wave budget; the waves of a set (group_waves.h) run as ONE persistent tcgen05 stage-1 launch over
+// all their work items (the device wave table, umma_stage1_waves), the normaliser per wave, and ONE stage-2
 // launch over all their columns (launch_stage2_waves).  A wave's stage-1 tiles are aligned (64
 // rows, 128 columns) and may take in a neighbouring group's rows or particles, which its stage 2
 // then leaves out.
@@ -1684,10 +1685,9 @@ int search_mdomain_groups(pftcc_handle *h, int ngroups, const int *ref0, const i
         const int st = umma_reset(h);    // the device error word of the bounded waits (allocated once)
         if (st != PFTCC_OK) return st;
     }
-    // a wave's packed spectrum within 1 GiB; a batch's waves within 2 GiB of Z and 1 GiB of factors
-    // at a time
-    const size_t z_wave_max = 1ull << 30, z_batch_max = 2ull << 30, d_batch_max = 1ull << 30;
-    struct WavePlan { int r_lo, r_hi, a_lo, a_hi, c_lo, c_hi, t_lo, t_hi; };
+    // a wave's packed spectrum within 1 GiB; a set's waves within 2 GiB of Z and 1 GiB of factors
+    const size_t z_wave_max = 1ull << 30, z_set_max = 2ull << 30, d_set_max = 1ull << 30;
+    const WaveGeom wg{P, ns, dlen, J, S1_TILE, COL_TILE};
     int cur_par = -1;
     for (const Batch &bt : batches) {
         const int par = bt.par;
@@ -1724,34 +1724,17 @@ int search_mdomain_groups(pftcc_handle *h, int ngroups, const int *ref0, const i
         for (int q = bt.q0; q < bt.q1; ++q) {
             const int c_lo = cb[2 * q + par] - bt.c0, c_hi = ce[2 * q + par] - bt.c0;
             if (c_hi <= c_lo) continue;
-            const int t_lo = c_lo / COL_TILE, t_hi = (c_hi + COL_TILE - 1) / COL_TILE;
-            const size_t zcol = (size_t)(t_hi - t_lo) * COL_TILE * P * sizeof(float2);   // Z bytes per row
-            int rows_max = (int)std::max<size_t>(S1_TILE, z_wave_max / zcol / S1_TILE * S1_TILE);
-            for (int r_lo = ref0[q] * ns, r_end = (ref0[q] + nref[q]) * ns; r_lo < r_end;) {
-                const int a_lo = r_lo / S1_TILE * S1_TILE;
-                const int r_hi = std::min(r_end, a_lo + rows_max);
-                const int a_hi = (r_hi + S1_TILE - 1) / S1_TILE * S1_TILE;
-                plan.push_back(WavePlan{r_lo, r_hi, a_lo, a_hi, c_lo, c_hi, t_lo, t_hi});
-                r_lo = r_hi;
-            }
+            plan_waves(plan, wg, ref0[q] * ns, (ref0[q] + nref[q]) * ns, c_lo, c_hi, z_wave_max);
         }
         // sets of waves: one stage-1 launch, the normalisers, one stage-2 launch each
         for (size_t w0 = 0; w0 < plan.size();) {
-            size_t zb = 0, db = 0, yb = 0, w1 = w0;
-            while (w1 < plan.size()) {
-                const WavePlan &p = plan[w1];
-                const size_t z = (size_t)P * (p.a_hi - p.a_lo) * (p.t_hi - p.t_lo) * COL_TILE * sizeof(float2);
-                const int nrw = (p.r_hi - 1) / ns - p.r_lo / ns + 1;
-                const size_t d = (size_t)nrw * (p.c_hi - p.c_lo) * dlen * sizeof(float);
-                const size_t y = (size_t)nrw * (p.c_hi - p.c_lo) * J * sizeof(float2);
-                if (w1 > w0 && (zb + z > z_batch_max || db + d > d_batch_max)) break;
-                zb += z; db += d; yb = std::max(yb, y); ++w1;
-            }
-            int st = ensure(h, (void **)&ws.X, &ws.X_elems, zb, "grouped Z");
+            WaveBytes sum;
+            const size_t w1 = wave_set_end(plan, w0, wg, z_set_max, d_set_max, &sum);
+            int st = ensure(h, (void **)&ws.X, &ws.X_elems, sum.z, "grouped Z");
             if (st) return st;
-            st = ensure(h, (void **)&ws.D, &ws.D_bytes, db, "grouped factors");
+            st = ensure(h, (void **)&ws.D, &ws.D_bytes, sum.d, "grouped factors");
             if (st) return st;
-            st = ensure(h, (void **)&ws.Yn, &ws.Y_bytes, yb, "grouped Y");
+            st = ensure(h, (void **)&ws.Yn, &ws.Y_bytes, sum.y, "grouped Y");
             if (st) return st;
             std::vector<S1Wave> s1;
             std::vector<S2Wave> s2;
@@ -1777,8 +1760,9 @@ int search_mdomain_groups(pftcc_handle *h, int ngroups, const int *ref0, const i
                                 ws.Yn, Dw, 1.0 / (2.0 * N), 0), "norm");
                 s2.push_back(S2Wave{Xw, Dw, p.r_lo, p.r_hi - p.r_lo, p.r_lo - p.a_lo, xrows, xcols, p.c_lo, cols,
                                     p.c_lo - p.t_lo * COL_TILE, r_lo_ref, cols, 0, 0});
-                zo += (size_t)P * xrows * xcols * sizeof(float2);
-                dof += (size_t)nrw * cols * dlen * sizeof(float);
+                const WaveBytes used = wave_bytes(wg, p);
+                zo += used.z;
+                dof += used.d;
             }
             if (precision == PFTCC_PREC_BF16X3) {
                 st = umma_stage1_waves(h, M, s1);

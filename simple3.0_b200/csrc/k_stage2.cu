@@ -826,7 +826,8 @@ static cudaError_t launch_s2(pftcc_handle *h, const S2Fast &sp, int blocks, cons
 }
 
 // every wave of the list in one launch, one block per column (blk0 filled in); rot: the candidates
-// carry their rotation (nothing re-scores them)
+// carry their rotation (nothing re-scores them).  The waves are in column order and share no column: a block
+// merges its rows into its column's top 8 with no order between blocks
 cudaError_t launch_stage2_waves(pftcc_handle *h, int P, std::vector<S2Wave> &waves, int nshifts, int nrs_total,
                                 float2 *cand, float *ccall, const int *perm, int eu, int rot)
 {
@@ -834,12 +835,14 @@ cudaError_t launch_stage2_waves(pftcc_handle *h, int P, std::vector<S2Wave> &wav
     const int nw = (int)waves.size();
     if (nw == 0) return cudaSuccess;
     long long blocks = 0;
+    int next_col = 0;
     for (S2Wave &w : waves) {
-        if ((unsigned long long)P * w.xcols * w.xrows >= (1ull << 32) || w.cols <= 0 || w.rows <= 0 ||
+        if (w.col0 < next_col || (unsigned long long)P * w.xcols * w.xrows >= (1ull << 32) || w.cols <= 0 || w.rows <= 0 ||
             w.zc0 + w.cols > w.xcols || w.rofs + w.rows > w.xrows || (w.xrows & 1))
             return cudaErrorInvalidValue;
         w.blk0 = (int)blocks;
         blocks += w.cols;
+        next_col = w.col0 + w.cols;
     }
     if (blocks >= (1LL << 31)) return cudaErrorInvalidValue;
     if (us.s2waves_cap < nw) {

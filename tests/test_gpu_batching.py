@@ -135,3 +135,29 @@ def test_grouped_search_captured_in_a_graph(pkg):
     finally:
         torch.cuda.synchronize()
         pc2.kill()
+
+
+@pytest.mark.parametrize("make,nrefs,nptcls", [("config0", 200, 500), ("config1", 100, 250)])
+@pytest.mark.parametrize("precision", ["bf16x3", "fp32"])
+def test_group_cut_by_rows_equals_the_ungrouped_search(pkg, make, nrefs, nptcls, precision):
+    """a group whose packed spectrum passes a wave's budget (81 shifts: 16,200 and 8,100 rows) is cut by
+    rows, its waves all merging into the same particles' candidates: the best over all of its rows,
+    bit for bit as the ungrouped search finds it, every time"""
+    w = getattr(pkg.synth, make)(nrefs=nrefs, nptcls=nptcls)
+    refs, R = pkg.synth.make_refs(w)
+    parts = pkg.synth.make_particles(w, R)
+    s = (np.arange(9) - 4.0) * 0.5
+    shifts = np.stack(np.meshgrid(s, s, indexing="ij"), -1).reshape(-1, 2).astype(np.float32)
+    pc = pkg.polarft_corrcalc()
+    pc.new(nrefs, (1, nptcls), box=w.box, nrots=w.nrots, kfromto=(w.kfrom, w.kto), ctf=True, ctf_frame="ptcl",
+           eoarr=[i % 2 for i in range(nptcls)])
+    pc.set_refs(1, refs.numpy(), True)
+    pc.set_refs(1, refs.numpy() * np.complex64(0.8 + 0.2j), False)
+    pc.polarize_ptcls(0, parts.cmat.numpy())
+    pc.create_polar_absctfmats(pkg.ctfparams_array(nptcls, smpd=w.smpd, kv=w.kv, cs=w.cs, fraca=w.fraca,
+                                                   dfx=parts.dfx, dfy=parts.dfy, angast=parts.angast))
+    for ntop in (0, 8):
+        want = pc.search_best(shifts, precision, ntop=ntop).copy()
+        for _ in range(3):
+            _same(pc.search_groups([(1, nrefs, 1, nptcls)], shifts, precision, ntop=ntop), want)
+    pc.kill()
