@@ -2,9 +2,8 @@
 // handle life cycle, host-side tables (polar grid, shift constants, gridding taps),
 // setters/getters and the per-pair and batched correlation entry points.
 #include "pftcc_internal.cuh"
+#include "download.h"
 
-#include <system_error>
-#include <thread>
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -1643,55 +1642,54 @@ int pftcc_calc_roinv_corrmat(pftcc_handle *h, float *corrmat)
 
 }  // extern "C"
 
-// A large result into the caller's pageable memory: pieces through two pinned buffers, the next piece on its
-// way while this one is copied out by a few threads (which also take the page faults of fresh memory side
-// by side).  One pageable copy of 51 MB took 10.7 ms of corr_all's 13.2, this takes 4.5.  Below
-// two pieces the plain copy is as fast.
-constexpr size_t DL_PIECE = 4u << 20;
-constexpr int DL_THREADS = 4;
+// the device side of a download on the handle's stream (download.h)
+struct HandleDownload {
+    pftcc_handle *h;
+    const char *src_dev, *what;
+    const void *dst;
 
-static void copy_out(char *dst, const char *src, size_t bytes)
-{
-    std::thread th[DL_THREADS - 1];
-    const size_t part = (bytes / DL_THREADS + 4095) & ~size_t(4095);
-    int started = 0;
-    try {
-        for (; started < DL_THREADS - 1 && (started + 1) * part < bytes; ++started) {
-            const size_t o = (started + 1) * part;
-            th[started] = std::thread([=] { std::memcpy(dst + o, src + o, std::min(part, bytes - o)); });
-        }
-    } catch (const std::system_error &) {   // no more threads: the rest here
+    bool pageable() const
+    {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, dst) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+        cudaGetLastError();   // not sticky
+        return false;
     }
-    std::memcpy(dst, src, std::min(part, bytes));
-    const size_t o = (size_t)(started + 1) * part;
-    if (o < bytes) std::memcpy(dst + o, src + o, bytes - o);
-    for (int i = 0; i < started; ++i) th[i].join();
-}
-
-static int download(pftcc_handle *h, void *dst, const void *src_dev, size_t bytes, const char *what)
-{
-    if (bytes < 2 * DL_PIECE) {
-        CK(cudaMemcpyAsync(dst, src_dev, bytes, cudaMemcpyDeviceToHost, h->stream), what);
+    char *piece(int i)
+    {
+        if ((!h->dl_buf[i] && cudaMallocHost(&h->dl_buf[i], DL_PIECE) != cudaSuccess) ||
+            (!h->dl_ev[i] && cudaEventCreateWithFlags(&h->dl_ev[i], cudaEventDisableTiming) != cudaSuccess)) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return static_cast<char *>(h->dl_buf[i]);
+    }
+    int copy(void *to, size_t offset, size_t n)
+    {
+        CK(cudaMemcpyAsync(to, src_dev + offset, n, cudaMemcpyDeviceToHost, h->stream), what);
+        return PFTCC_OK;
+    }
+    int mark(int i)
+    {
+        CK(cudaEventRecord(h->dl_ev[i], h->stream), what);
+        return PFTCC_OK;
+    }
+    int wait(int i)
+    {
+        CK(cudaEventSynchronize(h->dl_ev[i]), what);
+        return PFTCC_OK;
+    }
+    int sync()
+    {
         CK(cudaStreamSynchronize(h->stream), what);
         return PFTCC_OK;
     }
-    for (int i = 0; i < 2; ++i) {
-        if (!h->dl_buf[i]) CK(cudaMallocHost(&h->dl_buf[i], DL_PIECE), what);
-        if (!h->dl_ev[i]) CK(cudaEventCreateWithFlags(&h->dl_ev[i], cudaEventDisableTiming), what);
-    }
-    const size_t n = (bytes + DL_PIECE - 1) / DL_PIECE;
-    auto size = [&](size_t i) { return std::min(DL_PIECE, bytes - i * DL_PIECE); };
-    for (size_t i = 0; i <= n; ++i) {
-        if (i < n) {   // the buffer was copied out two pieces ago
-            CK(cudaMemcpyAsync(h->dl_buf[i & 1], static_cast<const char *>(src_dev) + i * DL_PIECE, size(i),
-                               cudaMemcpyDeviceToHost, h->stream), what);
-            CK(cudaEventRecord(h->dl_ev[i & 1], h->stream), what);
-        }
-        if (i == 0) continue;
-        CK(cudaEventSynchronize(h->dl_ev[(i - 1) & 1]), what);
-        copy_out(static_cast<char *>(dst) + (i - 1) * DL_PIECE, static_cast<const char *>(h->dl_buf[(i - 1) & 1]), size(i - 1));
-    }
-    return PFTCC_OK;
+};
+
+static int download(pftcc_handle *h, void *dst, const void *src_dev, size_t bytes, const char *what)
+{
+    HandleDownload d{h, static_cast<const char *>(src_dev), what, dst};
+    return download(d, static_cast<char *>(dst), bytes);
 }
 
 extern "C" {

@@ -79,3 +79,16 @@ def test_zero_reference_is_never_the_best(pkg):
     best = pc.search_best(None, "exact")
     assert np.all(best["iref"] == 0) and np.all(best["irot"] == 0) and np.all(np.isneginf(best["corr"]))
     pc.kill()
+
+
+def test_large_result_into_page_locked_memory(pkg):
+    """9.8 MB of correlations: page-locked and pageable destinations hold the same"""
+    import ctypes as C
+
+    import torch
+    w, pc, refs = build(pkg, "config0", 64, 300, "ref")
+    want = pc.corr_all(None)
+    got = torch.zeros(want.shape, dtype=torch.float32).pin_memory()
+    pc._check(pc._L.pftcc_corr_all(pc._h, 0, None, C.cast(got.data_ptr(), C.POINTER(C.c_float))))
+    assert np.array_equal(got.numpy(), want)
+    pc.kill()
