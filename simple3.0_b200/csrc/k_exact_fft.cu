@@ -14,6 +14,9 @@
 // reference and one of the particle are multiplied, the products summed over the pairs in registers,
 // and one transform of the sums gives every rotation: R(s) = (1/P) sum_j T(j) w_P^{-js}.
 //
+// A normaliser that is small beside the squares it is made of (the reference's energy lies where the CTF
+// almost vanishes) is within the transforms' rounding; it is formed term by term instead (ex_direct_norm).
+//
 // Operands are prepared as k_exact prepares them (FP32 products with the FP32-rounded shift phases
 // of the FP64 recurrence); everything after that is FP64, as there: measured on the cases' ranges
 // against 64-bit results the error is that of the final FP32 rounding (5e-8 to 9e-8), as before.
@@ -87,6 +90,23 @@ __device__ __forceinline__ pftcc_best ex_best(const Work *work, int first, float
     return b;
 }
 
+// D(s) = sum_k sum_n |ref(k, n)|^2 CTF^2(k, n + s) term by term, s < P.  The transforms leave D with an error
+// of a few 2^-53 of B = sum over the shell pairs of (sum_n of both shells' |ref|^2) (sum_n of both shells'
+// CTF^2): by Cauchy-Schwarz they round at eps |a|_2 |b|_2 a pair, and the squares are not negative.  Above 1e-7 B
+// that is 1e-8 of D at most, 5e-9 of a correlation (2^-24, its rounding, is 6e-8); below it this takes over.
+__device__ __noinline__ double ex_direct_norm(const float2 *ref, const float *sn, const float *ctf, int Ks, int P, int s)
+{
+    double d = 0.0;
+    for (int ik = 0; ik < Ks; ++ik)
+        for (int n = 0; n < P; ++n) {
+            float2 v = ref[ik * P + n];
+            if (sn) { v.x *= sn[ik]; v.y *= sn[ik]; }
+            const float c = ctf ? ctf[ik * P + (n + s < P ? n + s : n + s - P)] : 1.f;
+            d = fma((double)fmaf(v.x, v.x, __fmul_rn(v.y, v.y)), (double)(c * c), d);
+        }
+    return d;
+}
+
 // One block takes `per` items of one group, R at a time, G shell pairs per iteration:
 //   stage   every item's prepared samples and the particle's, 2 G shells, into shared memory
 //   pass 1  task (transform, n1): a length-P2 DFT over n2 of the channel's sequence, times the twiddles
@@ -111,6 +131,7 @@ __global__ void __launch_bounds__(T, MB) k_exact_fft(const __grid_constant__ ExA
     float *stg2 = reinterpret_cast<float *>(stg + (R + 1) * KK * P);   // [R + 1][KK][P] squares
     double *W = reinterpret_cast<double *>(stg + (R + 1) * KK * P);    // [K] Euclidean shell weights (no squares then)
     __shared__ double sums[R + 1];
+    __shared__ double dmag[R];    // B of ex_direct_norm
     __shared__ float imax[R];
     __shared__ float bcc[T / 32];
     __shared__ int bit[T / 32], brt[T / 32];
@@ -165,6 +186,7 @@ __global__ void __launch_bounds__(T, MB) k_exact_fft(const __grid_constant__ ExA
         double2 acc[NACC];
 #pragma unroll
         for (int i = 0; i < NACC; ++i) acc[i] = make_double2(0.0, 0.0);
+        double mag = 0.0;   // B, of item t < R
         // cc_2 sums the reference's squares over all shells, cc_1 to kstop; the Euclidean sums to kstop
         for (int k0 = 0; k0 < K; k0 += KK) {
             const bool spectra = k0 < Ks;
@@ -284,6 +306,13 @@ __global__ void __launch_bounds__(T, MB) k_exact_fft(const __grid_constant__ ExA
                     acc[i].y = fma(a.y, b.x, fma(-a.x, b.y, acc[i].y));
                 }
             }
+            if (CH == 3 && t < R) {
+#pragma unroll
+                for (int gq = 0; gq < G; ++gq) {   // j = 0: the sums of the pair's two shells
+                    const double2 a = buf[(size_t)((t * G + gq) * CH + 2) * ROW], b = buf[(size_t)((R * G + gq) * CH + 2) * ROW];
+                    mag = fma(a.x + a.y, b.x + b.y, mag);
+                }
+            }
             // the next iteration's barrier after the staging keeps pass 1 off the rows still read here
         }
         __syncthreads();
@@ -301,7 +330,10 @@ __global__ void __launch_bounds__(T, MB) k_exact_fft(const __grid_constant__ ExA
             const int e = t + i * T, f = e / P, j = e % P, k2 = j / P1, k1 = j % P1;
             if (f < R * CH) buf[(size_t)f * ROW + k2 + P2 * k1] = acc[i];
         }
-        if (t < R) imax[t] = -INFINITY;
+        if (t < R) {
+            imax[t] = -INFINITY;
+            dmag[t] = mag;
+        }
         __syncthreads();
         for (int r = t >> 5; r <= R; r += T / 32) {
             double s = 0.0;
@@ -351,10 +383,17 @@ __global__ void __launch_bounds__(T, MB) k_exact_fft(const __grid_constant__ ExA
             } else {
                 double d = sums[r];
                 if (FRAME == PFTCC_FRAME_PTCL) {
-                    // a D that vanishes (no sample where neither |ref| nor the CTF is zero) is left by the
-                    // transforms as rounding of the square sums, 1e-16 of them: 0 / 0 as the direct sums have it
                     d = buf[(size_t)(r * CH + CH - 1) * ROW + at].x / P;
-                    if (d <= 1e-14 * sums[r]) d = NAN;
+                    if (d <= 1e-7 * dmag[r]) {
+                        const int iref = x.one ? x.one_work.iref : x.work[grp.first + it0 + r].iref;
+                        d = dmag[r] == 0.0 ? 0.0
+                                           : ex_direct_norm(refs + (long long)iref * K * P,
+                                                            x.snorm ? x.snorm + ((size_t)(even ? 0 : 1) * x.nrefs + iref) * Ks : nullptr,
+                                                            ctf, Ks, P, s);
+                        // no sample where neither |ref| nor the CTF is zero: 0 / 0 as the direct sums have it, the
+                        // numerator being left as rounding
+                        if (d == 0.0) d = NAN;
+                    }
                 }
                 const double den = sqrt(d * sqp);
                 c0 = (float)((ce + co) / den);

@@ -81,6 +81,73 @@ def test_zero_reference_is_never_the_best(pkg):
     pc.kill()
 
 
+def test_weak_ctf(pkg, O):
+    """|CTF| of 4e-9 at most (defocus 1e-10 um, no spherical aberration or amplitude contrast): the correlations
+    are those of any multiple of it.  It is stored in FP32, off by a few 2^-24 a sample: 1e-6"""
+    w = pkg.synth.config0(nrefs=5, nptcls=3)
+    refs, R = pkg.synth.make_refs(w)
+    parts = pkg.synth.make_particles(w, R)
+    pc = pkg.polarft_corrcalc()
+    pc.new(5, (1, 3), box=w.box, nrots=w.nrots, kfromto=(w.kfrom, w.kto), ctf=True, ctf_frame="ptcl", eoarr=[0] * 3)
+    pc.set_refs(1, refs.numpy(), True)
+    pc.polarize_ptcls(0, parts.cmat.numpy())
+    df = np.full(3, 1e-10, np.float32)
+    pc.create_polar_absctfmats(pkg.ctfparams_array(3, smpd=w.smpd, kv=w.kv, cs=0.0, fraca=0.0, dfx=df, dfy=df))
+    g = O.geom(w.nrots, w.kfrom, w.kto, w.box)
+    t = O.tables(g)
+    ctf = O.ctfmat(g, t, O.make_ctf(w.smpd, w.kv, 0.0, 0.0, 1e-10, 1e-10, 0.0))
+    assert 0 < ctf.max() < 1e-8
+    ptcls = np.stack([pc.get_ptcl_pft(i + 1) for i in range(3)])
+    want = O.allcorrs64(g, t, refs.numpy(), ptcls, np.stack([ctf] * 3) / ctf.max(), None, "ptcl")
+    assert np.max(np.abs(pc.corr_all(None) - want)) < 1e-6
+    assert np.max(np.abs(pc.search_best(None, "exact")["corr"] - want.reshape(3, -1).max(1))) < 1e-6
+    pc.kill()
+
+
+@pytest.mark.parametrize("name", ["config0", "config1", "geometry_c"])
+def test_reference_where_the_ctf_almost_vanishes(pkg, O, name):
+    """a reference on one shell, the defocus such that |CTF| is near 2e-6 there (and not on the shells it is
+    transformed with): the correlations times the particle's norm are those of a handle of that shell alone,
+    up to each value's rounding, the FP32 square sums (2^-24 and some each) and what the transforms leave: 3e-7"""
+    w = getattr(pkg.synth, name)(nrefs=1, nptcls=2)
+    refs, R = pkg.synth.make_refs(w)
+    parts = pkg.synth.make_particles(w, R)
+    k = w.kfrom + 6
+    g = O.geom(w.nrots, w.kfrom, w.kto, w.box)
+    t = O.tables(g)
+
+    def shell(df):
+        return np.median(O.ctfmat(g, t, O.make_ctf(w.smpd, w.kv, w.cs, w.fraca, float(df), float(df), 0.0))[k - w.kfrom])
+
+    dfs = np.arange(0.2, 12.0, 0.002)     # towards a zero of the shell's CTF, then to where FP32 defocus values give 2e-6
+    df = dfs[np.argmin([shell(x) for x in dfs])]
+    for step in (1e-4, 1e-5, 1e-6):
+        near = df + step * np.arange(-30, 31)
+        df = near[np.argmin([abs(shell(x) - 2e-6) for x in near])]
+    df = np.full(2, df, np.float32)
+    assert shell(df[0]) < 1e-5
+    one = np.zeros_like(refs.numpy())
+    one[:, k - w.kfrom] = refs.numpy()[:, k - w.kfrom]
+    got = []
+    ptcls = None
+    for lo, hi in ((w.kfrom, w.kto), (k, k)):
+        pc = pkg.polarft_corrcalc()
+        pc.new(1, (1, 2), box=w.box, nrots=w.nrots, kfromto=(lo, hi), ctf=True, ctf_frame="ptcl", eoarr=[0] * 2)
+        pc.set_refs(1, one[:, lo - w.kfrom:hi + 1 - w.kfrom], True)
+        if ptcls is None:
+            pc.polarize_ptcls(0, parts.cmat.numpy())
+            ptcls = np.stack([pc.get_ptcl_pft(i + 1) for i in range(2)])
+        else:
+            pc.set_ptcls(0, ptcls[:, k - w.kfrom:k + 1 - w.kfrom])
+        pc.create_polar_absctfmats(pkg.ctfparams_array(2, smpd=w.smpd, kv=w.kv, cs=w.cs, fraca=w.fraca, dfx=df, dfy=df))
+        norm = np.sqrt([np.float64(pc.get_sqsum_ptcl(i + 1)) for i in range(2)])
+        got.append(pc.corr_all(None).astype(np.float64)[:, 0, 0] * norm[:, None])
+        pc.kill()
+    assert np.all(np.isfinite(got[0]))
+    scale = np.abs(got[1]).max(1, keepdims=True)
+    assert np.max(np.abs(got[0] - got[1]) / scale) < 3e-7
+
+
 def test_large_result_into_page_locked_memory(pkg):
     """9.8 MB of correlations: page-locked and pageable destinations hold the same"""
     import ctypes as C
