@@ -3,6 +3,7 @@
 // setters/getters and the per-pair and batched correlation entry points.
 #include "pftcc_internal.cuh"
 #include "download.h"
+#include "unit_root.h"
 
 #include <algorithm>
 #include <cmath>
@@ -432,10 +433,7 @@ int pftcc_new(const pftcc_config *cfg, const int *ptcl_mask, const int *eoarr, p
         (st = alloc_ptcl_arrays(h)))
         return fail(st, h->last_err);
     std::vector<double2> wn(h->g.N);
-    for (int e = 0; e < h->g.N; ++e) {
-        const double a = -2.0 * M_PI * e / h->g.N;
-        wn[e] = make_double2(cos(a), sin(a));
-    }
+    for (int e = 0; e < h->g.N; ++e) unit_root(-e, h->g.N, &wn[e].x, &wn[e].y);
     if (cudaMemcpyAsync(h->d_wn, wn.data(), wn.size() * sizeof(double2), cudaMemcpyHostToDevice, h->stream) ||
         cudaMemsetAsync(h->refs_even, 0, (size_t)h->nrefs * KP * sizeof(float2), h->stream) ||
         cudaMemsetAsync(h->refs_odd, 0, (size_t)h->nrefs * KP * sizeof(float2), h->stream) ||
