@@ -95,8 +95,7 @@ __global__ void __launch_bounds__(POL_THREADS) k_polarize(Geom g, const float2 *
 cudaError_t launch_polarize(pftcc_handle *h, const float2 *cmats, int n, int first_slot)
 {
     const Geom &g = h->g;
-    // boxes whose half plane exceeds a block's shared memory are not served
-    if ((size_t)g.box * (g.box / 2 + 1) * sizeof(float2) > 227 * 1024) return cudaErrorInvalidValue;
+    if (!gridding_served(g.box)) return cudaErrorInvalidValue;
     if (n <= 0) return cudaErrorInvalidConfiguration;
     const size_t win = (size_t)(2 * g.kto + 3) * (g.kto + 2) * sizeof(float2);
     // images per block: as many as leave room for two blocks on an SM, or three of the largest windows in one

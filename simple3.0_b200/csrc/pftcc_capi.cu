@@ -259,6 +259,7 @@ static int build_polarizer(pftcc_handle *h, int griddev)
 {
     if (h->pol_griddev == griddev && h->pol_off) return PFTCC_OK;
     const Geom &g = h->g;
+    if (!gridding_served(g.box)) return PFTCC_OK;   // launch_polarize refuses; the offsets would not fit 16 bits
     const int N = g.N, P = g.P, K = g.K, KM = g.kto + 1, W = g.kto + 2, npts = K * P;
     std::vector<int16_t> off((size_t)npts * 9);
     std::vector<float> wt((size_t)npts * 9);

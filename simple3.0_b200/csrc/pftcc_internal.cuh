@@ -233,6 +233,10 @@ namespace pftcc {
 // the device's opt-in maximum (less the kernel's static shared memory) -- one fixed value,
 // so concurrent callers that launch the kernel with different sizes never lower the limit
 // under each other; cudaErrorInvalidValue when `bytes` exceeds it.
+// the boxes that gridding serves: those whose half plane fits a block's shared memory, 240 at most.  With
+// kto + 2 <= box / 2 (pftcc_new) the window that k_polarize stages, (2 kto + 3) (kto + 2) entries, then fits it too
+// and is addressed by 16-bit offsets and their complements (28,680 entries at box 240)
+inline bool gridding_served(int box) { return (size_t)box * (box / 2 + 1) * sizeof(float2) <= 227 * 1024; }
 cudaError_t smem_limit(const void *kernel, size_t bytes);
 
 int set_err(pftcc_handle *h, int code, const std::string &msg);
