@@ -10,7 +10,6 @@
 #include "pftcc_internal.cuh"
 
 #include <algorithm>
-#include <cstddef>
 #include <cmath>
 
 namespace pftcc {
@@ -483,8 +482,8 @@ cudaError_t launch_exact(pftcc_handle *h, const Group *groups, int ngroups, cons
                          const uint8_t *rotmask)
 {
     if (frame == FRAME_EUCLID && (!h->d_sig2 || !h->d_pxls)) return cudaErrorInvalidValue;
-    // the transforms wherever their lengths allow (tens of times fewer operations, no size at which the
-    // direct sums were faster); the direct sums serve the other numbers of rotations
+    // the transforms where they are instantiated, for 128, 360 and 600 rotations (tens of times fewer operations,
+    // no size at which the direct sums were faster); the direct sums serve every other number
     if (exact_fft_supported(h->g.P))
         return launch_exact_fft(h, groups, ngroups, work, shifts, mode, frame, cc1_kstop, max_items, out, best, rotmask,
                                 nullptr);
@@ -506,9 +505,6 @@ cudaError_t launch_exact(pftcc_handle *h, const Group *groups, int ngroups, cons
 // (:1863-1925), both branches (match_filt: unweighted sums normalised with
 // sqsums over kstop; otherwise shell weights k in numerator and both norms).
 // The drop-in calls and the shift search: the stored |CTF| matrices, one block per request.
-struct RotReq { int iref, slot, irot, ctf_mode; double sx, sy, ddf; };
-static_assert(sizeof(RotReq) == sizeof(RotReqH) && offsetof(RotReq, sx) == offsetof(RotReqH, sx),
-              "RotReqH mirrors RotReq");
 
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double *red)
@@ -589,32 +585,23 @@ __global__ void __launch_bounds__(FR_THREADS) k_for_rot(
     }
 }
 
-cudaError_t launch_for_rot(pftcc_handle *h, int iref, int slot, double sx, double sy, int irot, int match_filt,
-                           int want_grad, double ddf, double *out5)
+// n single-rotation requests already on the device
+cudaError_t launch_rot_reqs(pftcc_handle *h, const RotReq *reqs_dev, int n, double *out5)
 {
-    // a single request: stage it through the small device buffer used for work items
-    RotReq rq{iref, slot, irot, 0, sx, sy, ddf};
-    (void)want_grad;
-    cudaError_t e = cudaMemcpyAsync(h->d_work, &rq, sizeof(rq), cudaMemcpyHostToDevice, h->stream);
-    if (e != cudaSuccess) return e;
     PFTCC_LAUNCH(h);
-    k_for_rot<<<1, FR_THREADS, 0, h->stream>>>(h->g, reinterpret_cast<const RotReq *>(h->d_work), h->refs_even,
-                                                h->refs_odd, h->ptcls, h->ctfmats, h->d_iseven, h->argtransf,
-                                                h->argtransf1, h->cfg.with_ctf && h->ctf_ready,
-                                                match_filt, snorm_ptr(h), h->nrefs, out5);
+    k_for_rot<<<n, FR_THREADS, 0, h->stream>>>(h->g, reqs_dev, h->refs_even, h->refs_odd, h->ptcls, h->ctfmats, h->d_iseven,
+                                                h->argtransf, h->argtransf1, h->cfg.with_ctf && h->ctf_ready,
+                                                h->cfg.match_filt, snorm_ptr(h), h->nrefs, out5);
     return cudaGetLastError();
 }
 
-// n single-rotation requests already on the device (reqs_dev: RotReq layout, see
-// pftcc_internal.cuh), out5 [n][5] = f, df/dsx, df/dsy, df/ddf, unused
-cudaError_t launch_rot_reqs(pftcc_handle *h, const void *reqs_dev, int n, double *out5)
+cudaError_t launch_for_rot(pftcc_handle *h, int iref, int slot, double sx, double sy, int irot, double *out5)
 {
-    PFTCC_LAUNCH(h);
-    k_for_rot<<<n, FR_THREADS, 0, h->stream>>>(h->g, reinterpret_cast<const RotReq *>(reqs_dev), h->refs_even,
-                                                h->refs_odd, h->ptcls, h->ctfmats, h->d_iseven, h->argtransf,
-                                                h->argtransf1, h->cfg.with_ctf && h->ctf_ready,
-                                                h->cfg.match_filt, snorm_ptr(h), h->nrefs, out5);
-    return cudaGetLastError();
+    // a single request: stage it through the small device buffer used for work items
+    const RotReq rq{iref, slot, irot, 0, sx, sy};
+    cudaError_t e = cudaMemcpyAsync(h->d_work, &rq, sizeof(rq), cudaMemcpyHostToDevice, h->stream);
+    if (e != cudaSuccess) return e;
+    return launch_rot_reqs(h, reinterpret_cast<const RotReq *>(h->d_work), 1, out5);
 }
 
 // ---------------------------------------------------------------------------
@@ -862,7 +849,7 @@ __global__ void k_grad_reqs(const pftcc_grad_req *__restrict__ in, const int *__
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const pftcc_grad_req r = in[i];
-    out[i] = RotReq{r.iref - 1, slots[i], r.irot, 1, r.sx, r.sy, r.ddf};
+    out[i] = RotReq{r.iref - 1, slots[i], r.irot, 0, r.sx, r.sy};
     if (with_ctf) rctf[i] = rot_ctf(ctfp[slots[i]], r.ddf);
 }
 

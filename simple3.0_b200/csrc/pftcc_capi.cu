@@ -1430,7 +1430,7 @@ static int for_rot_common(pftcc_handle *h, int iref, int iptcl, double sx, doubl
         return euclid_single(h, iref, iptcl, sx, sy, irot, out5);
     }
     ST(ensure_small(h, 1, 1, h->g.N, 1));
-    CK(launch_for_rot(h, iref - 1, slot, sx, sy, irot, h->cfg.match_filt, 1, 0.0, h->d_dout), "for_rot kernel");
+    CK(launch_for_rot(h, iref - 1, slot, sx, sy, irot, h->d_dout), "for_rot kernel");
     CK(cudaMemcpyAsync(out5, h->d_dout, 5 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "for_rot");
     CK(cudaStreamSynchronize(h->stream), "for_rot");
     return PFTCC_OK;

@@ -273,15 +273,15 @@ bool exact_fft_supported(int P);
 cudaError_t launch_exact_fft(pftcc_handle *h, const Group *groups, int ngroups, const Work *work, const float *shifts,
                              int mode, int frame, int cc1_kstop, int max_items, float *out, pftcc_best *best,
                              const uint8_t *rotmask, const ExactOne *one);
-// single-rotation correlation requests: iref 0-based, slot, irot 1-based, ctf_mode 0 = the stored
-// |CTF| matrices (k_for_rot, the drop-in calls), 1 = |CTF| recomputed at defocus + ddf (k_adjoint); out5 [n][5] = f, df/dsx, df/dsy, df/ddf, unused
-struct RotReqH { int iref, slot, irot, ctf_mode; double sx, sy, ddf; };
-cudaError_t launch_rot_reqs(pftcc_handle *h, const void *reqs_dev, int n, double *out5);
-cudaError_t launch_for_rot(pftcc_handle *h, int iref, int slot, double sx, double sy, int irot,
-                           int match_filt, int want_grad, double ddf, double *out5);
+// single-rotation correlation requests, iref 0-based, slot, irot 1-based, with the stored |CTF| matrices
+// (k_for_rot: the drop-in calls and the shift search); out5 [n][5] = f, df/dsx, df/dsy, 0, unused
+struct RotReq { int iref, slot, irot, pad; double sx, sy; };
+cudaError_t launch_rot_reqs(pftcc_handle *h, const RotReq *reqs_dev, int n, double *out5);
+cudaError_t launch_for_rot(pftcc_handle *h, int iref, int slot, double sx, double sy, int irot, double *out5);
+// the adjoint, with |CTF| recomputed at defocus + ddf (k_adjoint); out5 [n][5] = f, df/dsx, df/dsy, df/ddf, unused
 size_t grad_work_bytes(int nreq);   // of h->d_work for launch_grad_batch
 cudaError_t launch_grad_batch(pftcc_handle *h, const pftcc_grad_req *req_dev, const int *slots_dev, int nreq,
-                              double *out4);
+                              double *out5);
 cudaError_t launch_zero_beyond_kstop(pftcc_handle *h);
 
 // k_exact frame of the Euclidean objective: reference frame with shell weights

@@ -238,7 +238,7 @@ int shsrch_batch(pftcc_handle *h, int mode, const pftcc_shsrch_opts &o, int n, c
 
     // ---- device buffers (small per-call areas, grown on demand)
     std::vector<int> who_rot, who_scan;
-    std::vector<RotReqH> rq;
+    std::vector<RotReq> rq;
     std::vector<EuclidReq> eq;
     std::vector<Work> work;
     std::vector<Group> groups;
@@ -259,7 +259,7 @@ int shsrch_batch(pftcc_handle *h, int mode, const pftcc_shsrch_opts &o, int n, c
         // ROT: value and shift gradient per request
         if (!who_rot.empty()) {
             const int nr = (int)who_rot.size();
-            const size_t req_bytes = (size_t)nr * (eu ? sizeof(EuclidReq) : sizeof(RotReqH));
+            const size_t req_bytes = (size_t)nr * (eu ? sizeof(EuclidReq) : sizeof(RotReq));
             const size_t out_stride = eu ? 3 : 5;
             int st = ensure(h, (void **)&h->d_work, &h->work_cap, std::max<size_t>(req_bytes, 4096), "shsrch requests");
             if (st) return st;
@@ -280,11 +280,11 @@ int shsrch_batch(pftcc_handle *h, int mode, const pftcc_shsrch_opts &o, int n, c
                 rq.resize(nr);
                 for (int b = 0; b < nr; ++b) {
                     const Problem &p = pr[who_rot[b]];
-                    rq[b] = RotReqH{p.iref0, p.slot, p.rirot, 0, p.rx, p.ry, 0.0};
+                    rq[b] = RotReq{p.iref0, p.slot, p.rirot, 0, p.rx, p.ry};
                 }
                 if ((e = cudaMemcpyAsync(h->d_work, rq.data(), req_bytes, cudaMemcpyHostToDevice, h->stream)) != cudaSuccess)
                     return cuda_err(h, e, "shsrch upload");
-                if ((e = launch_rot_reqs(h, h->d_work, nr, h->d_dout)) != cudaSuccess) return cuda_err(h, e, "shsrch rot");
+                if ((e = launch_rot_reqs(h, reinterpret_cast<const RotReq *>(h->d_work), nr, h->d_dout)) != cudaSuccess) return cuda_err(h, e, "shsrch rot");
             }
             o5.resize((size_t)nr * out_stride);
             if ((e = cudaMemcpyAsync(o5.data(), h->d_dout, o5.size() * sizeof(double), cudaMemcpyDeviceToHost,
