@@ -44,6 +44,25 @@ def test_every_correlation(pkg, O, name, kstop, frame):
     pc.kill()
 
 
+@pytest.mark.parametrize("frame", ["ref", "ptcl"])
+@pytest.mark.parametrize("name,kstop", [("config0", 20), ("config0", 9), ("config1", 37), ("geometry_c", 60), ("geometry_c", 55)])
+def test_every_correlation_with_a_ctf(pkg, O, name, kstop, frame):
+    """the third channel with a CTF that varies over samples and shells.  The stored |CTF| are FP32 of FP32
+    arguments: chi, some 30 here, is off by up to 2^-24 chi and a few of its terms' roundings, 4e-6, at each sample
+    on its own, and a correlation of unit vectors moves by the root mean square of that over |CTF|: 1e-5"""
+    w, pc, refs = build(pkg, name, 5, 3, frame, kstop=kstop, ctf=True)
+    parts = pkg.synth.make_particles(w, pkg.synth.make_refs(w)[1])
+    g = O.geom(w.nrots, w.kfrom, w.kto, w.box, kstop=kstop)
+    t = O.tables(g)
+    ptcls = np.stack([pc.get_ptcl_pft(i + 1) for i in range(3)])
+    ctfs = np.stack([O.ctfmat(g, t, O.make_ctf(w.smpd, w.kv, w.cs, w.fraca, float(parts.dfx[i]), float(parts.dfy[i]),
+                                               float(parts.angast[i]))) for i in range(3)])
+    for shifts in (None, np.array([[0.0, 0.0], [1.5, -0.75], [-2.0, 2.0]], np.float32)):
+        want = O.allcorrs64(g, t, refs, ptcls, ctfs, shifts, frame)
+        assert np.max(np.abs(pc.corr_all(shifts) - want)) < 1e-5
+    pc.kill()
+
+
 @pytest.mark.parametrize("name", ["config0", "config1", "geometry_c"])
 @pytest.mark.parametrize("frame", ["ref", "ptcl"])
 @pytest.mark.parametrize("nrefs,nptcls,ns", [(1, 3, 0), (2, 3, 1), (3, 2, 1), (4, 2, 2), (9, 2, 1), (21, 1, 2), (7, 40, 1)])

@@ -75,6 +75,42 @@ def test_image_groups(pkg, n):
     every.kill()
 
 
+@pytest.mark.parametrize("box,kto,nrots,n", [(64, 20, 128, 1187), (128, 40, 360, 593), (128, 40, 360, 889),
+                                              (128, 40, 360, 890), (200, 60, 600, 593), (200, 60, 600, 889),
+                                              (200, 60, 600, 891), (240, 118, 360, 3)])
+def test_image_groups_against_the_oracle(pkg, O, box, kto, nrots, n):
+    """gridding with one to four images a block (from 592, 888 and 1184 images on; box 200's window leaves room
+    for three, box 240's largest for one), remainders of each, against the oracle's polarize: nine products
+    summed in FP32, at most 2^-24 (9 + 1) of the taps' moduli, and the weights' rounding: 2e-6 of the largest
+    sample.  The square sums: the FP32 sum of 2 K P squares in a tree after a thread's share, 1e-5 relative"""
+    rng = np.random.default_rng(n)
+    kfrom = kto - 5
+    img = (rng.standard_normal((n, box, box // 2 + 1)) + 1j * rng.standard_normal((n, box, box // 2 + 1))).astype(np.complex64)
+    pc = pkg.polarft_corrcalc()
+    pc.new(1, (1, n), box=box, nrots=nrots, kfromto=(kfrom, kto))
+    pc.polarize_ptcls(0, img)
+    g = O.geom(nrots, kfrom, kto, box)
+    t = O.tables(g)
+    for i in sorted({0, 1, 2, 3, n // 2, n - 4, n - 3, n - 2, n - 1} & set(range(n))):
+        want = O.polarize(g, t, img[i])
+        got = pc.get_ptcl_pft(i + 1)
+        assert np.max(np.abs(got - want)) < 2e-6 * np.max(np.abs(want))
+        assert abs(pc.get_sqsum_ptcl(i + 1) / np.sum(np.abs(want) ** 2) - 1) < 1e-5
+    pc.kill()
+
+
+@pytest.mark.parametrize("box,kto", [(242, 40), (258, 127)])
+def test_boxes_past_the_gridding_are_refused(pkg, box, kto):
+    """box 258's window would not be addressed by 16-bit offsets either"""
+    pc = pkg.polarft_corrcalc()
+    pc.new(1, (1, 1), box=box, nrots=128, kfromto=(2, kto))
+    img = np.zeros((1, box, box // 2 + 1), np.complex64)
+    for _ in range(2):
+        with pytest.raises(pkg.PftccError):
+            pc.polarize_ptcls(0, img)
+    pc.kill()
+
+
 @pytest.mark.parametrize("nrots,kstop", [(128, 20), (128, 2), (128, 5), (100, 20), (34, 20), (360, 40), (600, 60)])
 def test_adjoint_segments(pkg, nrots, kstop):
     """without a CTF the adjoint is the drop-in gradient (which keeps one segment)"""
