@@ -470,7 +470,7 @@ static cudaError_t launch_ex_k(pftcc_handle *h, const ExArgs &x, int ngroups, in
 }
 
 // Threads and blocks per SM: the FP64 transforms hold 60 to 80 registers of data, so a block has few
-// warps and the kernel waits on its own chains (FP64 pipe 20 % busy, 12.5 % occupancy at P = 180);
+// warps and the kernel waits on its own chains (at P = 180 FP64 pipe 22 %, issue slots 30 %, 12 warps an SM);
 // the shapes below are the fastest of 96 to 416 threads and 1 to 4 blocks, with 1 or 2 shell pairs at
 // once for four items.  36,000 triples (100 particles, 40 references, 9 shifts) of the exact search:
 //   P = 64:   0.55 ms (G = 2, 160 threads, 3 blocks); 0.58 (G = 1, 128); 0.66 (G = 2, 160, 1)

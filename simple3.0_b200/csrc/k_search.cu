@@ -225,8 +225,9 @@ __global__ void __launch_bounds__(SPEC_THREADS) k_spec_ptcl(
 // polar samples a(n, k) are formed exactly as in k_spec_ref (FP32 products with the
 // single-precision shift phases of the de Moivre recurrence), a batch of shells at a time
 // ([shell][n] in shared memory), the recurrence state kept per angular sample n.
-// wn: the table w_N^{-e}, e < N.  What bounds these kernels: the latency of the FP64 chains and the block's
-// barriers, with 40 to 96 KB of rows and samples a block.  T threads: about the larger pass's tasks of a batch
+// wn: the table w_N^{-e}, e < N.  What bounds these kernels: the references' (P = 180), the rows' way through shared
+// memory (L1 data path 78 % busy, FP64 pipe 29 %, issue slots 45 %); the particles' (P = 300), the loads and the
+// block's barriers with 16 warps an SM (L1 50 %, FP64 17 %, issue slots 28 %).  T threads: about the larger pass's tasks of a batch
 // (a thread per transform and P1 or P2, two transforms a shell pair for the references, three for the particles,
 // one for |ref|^2, four pairs), so that small blocks share an SM instead of idle warps meeting at the barriers;
 // the particles' blocks, two an SM by their memory, stay at 256 from P = 180 on (192 threads: 0.70 ms, not 0.64).
@@ -566,7 +567,8 @@ static cudaError_t launch_spec_r2(pftcc_handle *h, const Geom &g, const float2 *
 // stored as the packed spectrum of stage 2, Z(m) and Z(P - m) (make_z).  Block tile 64
 // cols x 64 rows, 256 threads with 4 x 4 complex micro-tiles per plane, the whole shell
 // range of both planes staged in shared memory (Ks <= 64).
-// What bounds it: the FP32 pipe.  Real and imaginary parts are staged apart, [shell][64] with the
+// What bounds it: no single unit -- the FMA pipe 55 % busy, the L1 data path 56 %, the issue slots 55 %, with
+// 16 warps an SM (79.9 KB a block) whose loads wait.  Real and imaginary parts are staged apart, [shell][64] with the
 // groups of four rows exchanged by the shell's low bits, so that the transposing stores (a warp takes 8
 // shells x 4 rows) and the 16-byte reads are free of bank conflicts -- the (re, im) pairs it held before
 // cost 32-way conflicts on the way in and 2-way on the way out, as long as the arithmetic -- and two
@@ -706,9 +708,11 @@ __global__ void k_norm_cvt(int n, int J, int Ks, int n_pad, const double2 *__res
 // particles, 4 warps; every thread takes the 8 references (their spectra read at one address per
 // warp) and the particles l + 32 q (q < 4) of its warp's 128 (coalesced reads), 32 accumulators.
 // Y[(rl * J + j) * ncols + cl] unscaled (the transform applies the weights wgt_j / P): a warp stores 256
-// consecutive bytes.  What bounds it: the FP32 pipe and the write of Y (8 B a value).  With the j of a pair
-// next to each other instead, every store left 8 bytes of a 32-byte sector to be filled by another block
-// much later: 500 references x 2000 particles, P = 180, Ks = 39: 1.78 ms before, 0.98 now (29 TFLOP/s).
+// consecutive bytes.  What bounds it: the dependent chains of
+// its 12 warps an SM (three blocks by their shared memory): issue slots 54 % used, FMA pipe 45 %, L1 41 %, DRAM 9 %.
+// With the j of a pair next to each other instead, every store left 8 bytes of a 32-byte sector to be filled by
+// another block much later: 500 references x 2000 particles, P = 180, Ks = 39: 1.78 ms before, 0.96 now
+// (30 TFLOP/s).
 constexpr int NY2_R = 8, NY2_C = 512, NY2_KC = 8;   // references, particles and shells per chunk of a block
 constexpr int NY2_CS = NY2_C + 2;                    // a chunk's row: from an even column (16-byte copies)
 constexpr size_t NY2_SMEM = 2 * (size_t)NY2_KC * NY2_CS * sizeof(float2);
@@ -897,9 +901,10 @@ template <int P> __device__ __forceinline__ int norm_slot(int l, int b)
 
 // A batch's factors meet in shared memory (over the rows, which pass 2 has in registers by then) and go
 // out as 16-byte stores: the lanes of a warp hold rotations that lie apart in stage 2's order.
-// What bounds it: reading Y and writing the factors (800 B a pair at P = 180).  1e6 pairs, P = 180: 1.15
-// ms before (a block per column, 8-byte reads of Y, 4-byte stores of the factors), 0.80 now; 486,000 at
-// P = 300 0.96 in six launches before, 1.07 now (worth it for Y's order: both kernels 3.03 before, 2.9 now).
+// What bounds it: the transforms' way through shared memory (L1 data path 70 % busy, issue slots 51 %, FP64 pipe
+// 30 %; DRAM 21 %).  1e6 pairs, P = 180: 1.15 ms before (a block per column, 8-byte reads of Y, 4-byte stores of
+// the factors), 0.80 now; 486,000 at P = 300 0.96 in six launches before, 1.08 now (worth it for Y's order: both
+// kernels 3.03 before, 2.48 now).
 constexpr int NORM_CB = 8;
 template <int N1, int N2> struct NormFft {
     static constexpr int H = N1 * N2, P = 2 * H, J = H + 1;
