@@ -360,11 +360,16 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_umma_stage1(const __grid_const
         long long tacc = 0;
         bool ok = true;
         const int N = 2 * P;
-        int wv = 0;
+        int wv = 0, wv_seen = -1;
         for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
             wave_of(up, w, wv);
             const S1Wave *W = up.waves + wv;
             const CUtensorMap *tmX = up.maps + wv;
+            // the map was copied to global memory since the last launch, at the address of an earlier launch's:
+            // the storing thread acquires it for the tensor-map proxy before its first use
+            if (lane == 0 && wv != wv_seen)
+                asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(tmX) : "memory");
+            wv_seen = wv;
             const int n_pt = __ldg(&W->n_ptiles), wi = w - __ldg(&W->item0);
             const int mp = wi / n_pt, pt = wi - mp * n_pt;
             const int n_rt = __ldg(&W->n_rtiles), xcols = __ldg(&W->xcols);

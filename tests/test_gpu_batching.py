@@ -161,3 +161,45 @@ def test_group_cut_by_rows_equals_the_ungrouped_search(pkg, make, nrefs, nptcls,
         for _ in range(3):
             _same(pc.search_groups([(1, nrefs, 1, nptcls)], shifts, precision, ntop=ntop), want)
     pc.kill()
+
+
+def test_group_cut_by_rows_captured_in_a_graph(pkg):
+    """the launches of a cut group follow one another inside a captured graph too: its replays give the
+    uncaptured call's result, bit for bit"""
+    import torch
+    nrefs, nptcls = 200, 300
+    w = pkg.synth.config0(nrefs=nrefs, nptcls=nptcls)
+    refs, R = pkg.synth.make_refs(w)
+    parts = pkg.synth.make_particles(w, R)
+    s = (np.arange(12) - 5.5) * 0.4          # 28,800 rows, 5,440 a wave: six launches
+    shifts = np.stack(np.meshgrid(s, s, indexing="ij"), -1).reshape(-1, 2).astype(np.float32)
+    side = torch.cuda.Stream()
+    pc = pkg.polarft_corrcalc()
+    pc.new(nrefs, (1, nptcls), box=w.box, nrots=w.nrots, kfromto=(w.kfrom, w.kto), ctf=False, ctf_frame="ptcl",
+           eoarr=[0] * nptcls)
+    pc.set_stream(side.cuda_stream)
+    pc.set_refs(1, refs.numpy(), True)
+    pc.polarize_ptcls(0, parts.cmat.numpy())
+    out = torch.zeros((nptcls, 4), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    args = ([(1, nrefs, 1, nptcls)], shifts, "bf16x3", 8, out.data_ptr())
+    pc.search_groups_dev(*args)
+    torch.cuda.synchronize()
+    pc.search_check()
+    want = out.clone()
+    _same(want.cpu().numpy().view([("iref", np.int32), ("irot", np.int32), ("ishift", np.int32), ("corr", np.float32)])[:, 0],
+          pc.search_best(shifts, "bf16x3", ntop=8))
+    pc.search_groups_dev(*args)               # sizes the workspace again after the other search
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):
+        pc.search_groups_dev(*args)
+    for _ in range(2):
+        out.zero_()
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    pc.search_check()
+    del g
+    pc.kill()
