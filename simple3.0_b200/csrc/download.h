@@ -4,8 +4,10 @@
 // Page-locked memory takes one direct copy.  A large result into pageable memory goes in pieces through
 // two pinned buffers, the next piece on its way while this one is copied out by a few threads (which
 // also take the page faults of fresh memory side by side): one pageable copy of 51 MB took 10.7 ms of
-// corr_all's 13.2, this takes 4.5.  Below two pieces the plain copy is as fast, and it serves where no pinned
-// memory is to be had.
+// corr_all's 13.2, this takes 4.5.  Below 32 MiB the plain copy is the faster: the allocator then gives back
+// pages that are already there, and there are no faults to share.  corr_all_prec into a new array, ms, through
+// the pieces and plain: 8 MiB 1.8 and 1.4, 16 MiB 2.8 and 2.5, 24 MiB 4.2 and 3.5, but 32 MiB 3.8 and 8.0, 64 MiB
+// 7.8 and 15.  The plain copy also serves where no pinned memory is to be had.
 //
 //   Dev::pageable()                false where the destination is page-locked (or not host memory)
 //   Dev::piece(i)                  pinned buffer i of 2, DL_PIECE bytes; null where there is none
@@ -23,6 +25,7 @@
 namespace pftcc {
 
 constexpr size_t DL_PIECE = 4u << 20;
+constexpr size_t DL_MIN = 32u << 20;   // the smallest result that goes in pieces
 constexpr int DL_THREADS = 4;
 
 inline void copy_out(char *dst, const char *src, size_t bytes)
@@ -46,7 +49,7 @@ inline void copy_out(char *dst, const char *src, size_t bytes)
 template <class Dev> int download(Dev &dev, char *dst, size_t bytes)
 {
     int st;
-    if (bytes < 2 * DL_PIECE || !dev.pageable() || !dev.piece(0) || !dev.piece(1)) {
+    if (bytes < DL_MIN || !dev.pageable() || !dev.piece(0) || !dev.piece(1)) {
         if ((st = dev.copy(dst, 0, bytes))) return st;
         return dev.sync();
     }

@@ -1,6 +1,6 @@
 """Host (CPU) tests of a large result's way to the caller (simple3.0_b200/csrc/download.h, built here with
 g++ over a device whose copies land when they are waited for): page-locked memory takes one direct copy,
-pageable memory pieces through two pinned buffers, the plain copy serves where there are none, and a
+a large result into pageable memory pieces through two pinned buffers, the plain copy serves where there are none, and a
 failed copy's status is returned."""
 import ctypes as C
 import os
@@ -11,7 +11,7 @@ import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "simple3.0_b200", "csrc")
-PIECE = 4 << 20
+PIECE, LARGE = 4 << 20, 32 << 20
 
 
 @pytest.fixture(scope="module")
@@ -32,10 +32,10 @@ def run(tmp_path_factory):
     return call
 
 
-@pytest.mark.parametrize("nbytes", [1, 4096, 2 * PIECE - 1, 2 * PIECE, 2 * PIECE + 1, 3 * PIECE + 4097, 5 * PIECE])
+@pytest.mark.parametrize("nbytes", [1, 2 * PIECE, LARGE - 1, LARGE, LARGE + 1, LARGE + PIECE + 4097])
 def test_route_and_contents(run, nbytes):
     n = -(-nbytes // PIECE)
-    large = nbytes >= 2 * PIECE
+    large = nbytes >= LARGE
     assert run(nbytes) == (0, n if large else 1, 0 if large else 1, True)
     assert run(nbytes, page_locked=True) == (0, 1, 1, True)
     for pieces in (0, 1):
@@ -44,5 +44,5 @@ def test_route_and_contents(run, nbytes):
 
 @pytest.mark.parametrize("fail", [0, 1, 2])
 def test_failed_copy(run, fail):
-    st, copies, _, _ = run(3 * PIECE, fail=fail)
+    st, copies, _, _ = run(LARGE, fail=fail)
     assert st == 7 and copies == fail + 1

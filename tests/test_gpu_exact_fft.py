@@ -168,11 +168,11 @@ def test_reference_where_the_ctf_almost_vanishes(pkg, O, name):
 
 
 def test_large_result_into_page_locked_memory(pkg):
-    """9.8 MB of correlations: page-locked and pageable destinations hold the same"""
+    """36 MB of correlations, past the 32 MiB that go in pieces: page-locked and pageable destinations hold the same"""
     import ctypes as C
 
     import torch
-    w, pc, refs = build(pkg, "config0", 64, 300, "ref")
+    w, pc, refs = build(pkg, "config0", 64, 1100, "ref")
     want = pc.corr_all(None)
     got = torch.zeros(want.shape, dtype=torch.float32).pin_memory()
     pc._check(pc._L.pftcc_corr_all(pc._h, 0, None, C.cast(got.data_ptr(), C.POINTER(C.c_float))))
