@@ -143,17 +143,17 @@ cudaError_t launch_sqsums(pftcc_handle *h, int first_slot, int n)
 // arithmetic: create_polar_absctfmats :926-935 (spaFreqSq from polar * 1/ldim,
 // ang = atan2(y, x)), simple_ctf.f90 constructor :54-70, init :73-81,
 // evalPhSh :88-98, eval_df :185-189, kV2wl :522-525, eval :147-153 / :154-160.
-// A block takes 256 samples of CTF_IMGS particles: the angle's arctangent once a sample, the optics'
+// A block takes 256 samples of I particles: the angle's arctangent once a sample, the optics'
 // constants once a particle, and per value one cosine and one sine.  What bounds it: those, then the
 // write of 4 B a value.  Before, with all of it per value: 5130 particles at box 200 1.04 ms, now 0.26.
 struct CtfF { float wl, cs, ampc, dfx, dfy, angast, phshift; int l_phaseplate; };
-constexpr int CTF_IMGS = 16;
 
+template <int I>
 __global__ void __launch_bounds__(256) k_ctfmat(Geom g, const float *__restrict__ polar,
                                                 const pftcc_ctfparams *__restrict__ params, int n, float *__restrict__ out)
 {
-    __shared__ CtfF cf[CTF_IMGS];
-    const int i0 = blockIdx.y * CTF_IMGS, ni = min(CTF_IMGS, n - i0);
+    __shared__ CtfF cf[I];
+    const int i0 = blockIdx.y * I, ni = min(I, n - i0);
     if ((int)threadIdx.x < ni) {
         const pftcc_ctfparams c = params[i0 + threadIdx.x];
         CtfF f;
@@ -192,11 +192,16 @@ __global__ void __launch_bounds__(256) k_ctfmat(Geom g, const float *__restrict_
 
 cudaError_t launch_ctfmat(pftcc_handle *h, const pftcc_ctfparams *params, int n, float *out)
 {
-    const int per = h->g.K * h->g.P;
-    dim3 grid((per + 255) / 256, (n + CTF_IMGS - 1) / CTF_IMGS);
+    // fewer particles a block where sixteen would leave less than four blocks, four less than two, for each of the 148
+    // SMs: 30 particles at box 64 17 us a call with one, 20 with sixteen (ten blocks of sixteen particles one after the other)
+    const int bx = (h->g.K * h->g.P + 255) / 256;
+    const long long blocks = (long long)n * bx;   // of one particle each
+    const int I = blocks >= 16 * 4 * 148 ? 16 : blocks >= 4 * 2 * 148 ? 4 : 1;
+    auto k = I == 16 ? k_ctfmat<16> : I == 4 ? k_ctfmat<4> : k_ctfmat<1>;
+    const dim3 grid(bx, (n + I - 1) / I);
     PFTCC_LAUNCH(h);
     KTimer kt(h, PFTCC_K_CTFMAT);
-    k_ctfmat<<<grid, 256, 0, h->stream>>>(h->g, h->polar, params, n, out);
+    k<<<grid, 256, 0, h->stream>>>(h->g, h->polar, params, n, out);
     return cudaGetLastError();
 }
 

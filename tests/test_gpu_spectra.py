@@ -47,9 +47,9 @@ def test_shell_batches(pkg, O, name, ks):
     pc.kill()
 
 
-@pytest.mark.parametrize("n", [1, 17, 1187])
+@pytest.mark.parametrize("n", [1, 17, 595, 1187, 1601])
 def test_image_groups(pkg, n):
-    """gridding takes up to four images a block, the CTF sixteen; box 48 with kto at its limit"""
+    """gridding takes up to four images a block, the CTF one, four or sixteen; box 48 with kto at its limit"""
     w = pkg.synth.config0(nrefs=1, nptcls=n)
     w.box, w.kto = 48, 22
     rng = np.random.default_rng(n)
